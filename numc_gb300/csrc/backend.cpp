@@ -178,6 +178,13 @@ struct Plan {
   int param;    // Rule8 for int8/uint8, FloatSimt for SIMT floats, slices for Ozaki
 };
 
+// A Plan's algorithm of 16-, 32- and 64-bit integers on the tensor cores (exact,
+// like the CUDA-core kernel): what the process-wide choice (SIMT, the only one
+// these dtypes have) runs where it is the faster one and the call has a
+// workspace.  Not a value of NumcCudaAlgo: NUMC_CUDA_ALGO_SIMT asked for by
+// number stays on the CUDA cores.
+constexpr int kAlgoIntDigits = 100;
+
 // numc_matmul_naive's arithmetic, passed as `param` by the library itself.
 constexpr int kParamNaive = -1000;
 
@@ -188,7 +195,8 @@ constexpr int kParamNaive = -1000;
 int resolve(NumcDType dt, int algo, int param, size_t M, size_t K, size_t N, Plan *p,
             bool packed_only = false) {
   ensure_algos();
-  if (algo == NUMC_CUDA_ALGO_DEFAULT) {
+  const bool by_default = algo == NUMC_CUDA_ALGO_DEFAULT;
+  if (by_default) {
     algo = g_algo[dt].algo.load();
     if (param == -1) param = g_algo[dt].param.load();
   }
@@ -254,6 +262,9 @@ int resolve(NumcDType dt, int algo, int param, size_t M, size_t K, size_t N, Pla
   }
   p->algo = algo;
   p->param = param;
+  if (by_default && algo == NUMC_CUDA_ALGO_SIMT && !isf && !is8 &&
+      numc_k::int_digits_workspace(dt, M, K, N))
+    p->algo = kAlgoIntDigits;
   if (isf && algo == NUMC_CUDA_ALGO_SIMT) {
     // numc's AVX-512 float kernels are not reproduced (their float64 packed
     // path overflows its stack buffer, gemm_avx512.h:278,797): the AVX-512
@@ -289,7 +300,8 @@ int resolve(NumcDType dt, int algo, int param, size_t M, size_t K, size_t N, Pla
   return 0;
 }
 
-size_t plan_workspace(const Plan &p, size_t M, size_t K, size_t N) {
+size_t plan_workspace(NumcDType dt, const Plan &p, size_t M, size_t K, size_t N) {
+  if (p.algo == kAlgoIntDigits) return numc_k::int_digits_workspace(dt, M, K, N);
   if (p.algo == NUMC_CUDA_ALGO_SPLIT_BF16) return numc_k::split_bf16_workspace(M, K, N, p.param);
   if (p.algo == NUMC_CUDA_ALGO_SPLIT_FP16) return numc_k::split_f16_workspace(M, K, N);
   if (p.algo == NUMC_CUDA_ALGO_OZAKI) return numc_k::ozaki_workspace(M, K, N, p.param);
@@ -307,6 +319,7 @@ int run_plan(NumcDType dt, const Plan &p, const numc_k::Gemm &g, void *ws,
   case NUMC_CUDA_ALGO_SPLIT_FP16: e = numc_k::launch_split_f16(g, p.param, ws, ws_bytes, s); break;
   case NUMC_CUDA_ALGO_OZAKI: e = numc_k::launch_ozaki(g, p.param, ws, ws_bytes, s); break;
   case NUMC_CUDA_ALGO_TC_INT8: e = numc_k::launch_int8_tc(dt, g, p.param, ws, ws_bytes, s); break;
+  case kAlgoIntDigits: e = numc_k::launch_int_digits(dt, g, ws, ws_bytes, s); break;
   }
   if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
   return 0;
@@ -329,20 +342,49 @@ int ctx_stream(NumcCtx *ctx, cudaStream_t *s) {
   return 0;
 }
 
-int ctx_scratch(NumcCtx *ctx, size_t bytes, cudaStream_t s, char **out) {
-  if (ctx->scratch_bytes < bytes) {
-    if (ctx->scratch) {
-      CU(cudaStreamSynchronize(s), "cudaStreamSynchronize");
-      cudaFree(ctx->scratch);
-      ctx->scratch = nullptr;
-      ctx->scratch_bytes = 0;
-    }
-    size_t grow = align_up(bytes + bytes / 4, 1 << 20);
-    CU(numc_k::dev_malloc(&ctx->scratch, grow), "cudaMalloc(scratch)");
-    ctx->scratch_bytes = grow;
+cudaError_t grow_scratch(NumcCtx *ctx, size_t bytes, cudaStream_t s) {
+  if (ctx->scratch_bytes >= bytes) return cudaSuccess;
+  cudaError_t e;
+  if (ctx->scratch) {
+    if ((e = cudaStreamSynchronize(s))) return e;
+    cudaFree(ctx->scratch);
+    ctx->scratch = nullptr;
+    ctx->scratch_bytes = 0;
   }
+  size_t grow = align_up(bytes + bytes / 4, 1 << 20);
+  if ((e = numc_k::dev_malloc(&ctx->scratch, grow))) return e;
+  ctx->scratch_bytes = grow;
+  return cudaSuccess;
+}
+
+int ctx_scratch(NumcCtx *ctx, size_t bytes, cudaStream_t s, char **out) {
+  CU(grow_scratch(ctx, bytes, s), "cudaMalloc(scratch)");
   *out = (char *)ctx->scratch;
   return 0;
+}
+
+// Scratch of `base` bytes for staged operands plus the plan's workspace
+// (*ws_bytes).  Integer plans give the tensor cores up for the CUDA cores,
+// which need no workspace, where the device has no room for the digits, where
+// the stream is being captured (the call then neither allocates nor reads the
+// status word), and, with an asynchronous result (`async`: a resident output and
+// inputs), where they would not save more than the status word's read costs the
+// caller (about 15 us).
+int plan_scratch(NumcCtx *ctx, NumcDType dt, Plan *plan, size_t M, size_t K, size_t N,
+                 size_t base, bool async, cudaStream_t s, size_t *ws_bytes, char **out) {
+  *ws_bytes = plan_workspace(dt, *plan, M, K, N);
+  if (plan->algo == kAlgoIntDigits) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool captured =
+        cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+    if (captured || (async && numc_k::int_digits_gain_us(dt, M, K, N) < 15) ||
+        grow_scratch(ctx, base + *ws_bytes + 256, s) != cudaSuccess) {
+      cudaGetLastError();
+      plan->algo = NUMC_CUDA_ALGO_SIMT;
+      *ws_bytes = 0;
+    }
+  }
+  return ctx_scratch(ctx, base + *ws_bytes + 256, s, out);
 }
 
 bool is_resident(const NumcArray *a) {
@@ -596,9 +638,10 @@ int matmul_impl(const NumcArray *a, const NumcArray *b, NumcArray *out, int algo
   size_t off_o = off_b + align_up(rb ? 0 : sb, 256);
   size_t off_bias = off_o + align_up(ro ? 0 : so, 256);
   size_t off_w = off_bias + align_up(rbias ? 0 : sbias, 256);
-  size_t ws_bytes = plan_workspace(plan, M, K, N);
+  size_t ws_bytes = 0;
   char *scratch = nullptr;
-  if ((err = ctx_scratch(ctx, off_w + ws_bytes + 256, s, &scratch))) return err;
+  if ((err = plan_scratch(ctx, dt, &plan, M, K, N, off_w, ra && rb && ro, s, &ws_bytes,
+                          &scratch))) return err;
 
   const char *da = ra ? a->dev_base : scratch + off_a;
   const char *db = rb ? b->dev_base : scratch + off_b;
@@ -624,7 +667,7 @@ int matmul_impl(const NumcArray *a, const NumcArray *b, NumcArray *out, int algo
   }
   // The fused epilogues add the bias themselves; the others get one pass.
   numc_k::Gemm gk = g;
-  if (!numc_k::fuses_bias(plan.algo)) gk.bias = nullptr;
+  if (plan.algo != kAlgoIntDigits && !numc_k::fuses_bias(plan.algo)) gk.bias = nullptr;
   if ((err = run_plan(dt, plan, gk, scratch + off_w, ws_bytes, s))) return err;
   if (g.bias && !gk.bias) {
     cudaError_t be = numc_k::launch_bias_add(dt, g, s);
@@ -641,7 +684,8 @@ int matmul_impl(const NumcArray *a, const NumcArray *b, NumcArray *out, int algo
     CU(cudaStreamSynchronize(s), "cudaStreamSynchronize");
   }
   if (plan.algo == NUMC_CUDA_ALGO_SPLIT_BF16 || plan.algo == NUMC_CUDA_ALGO_SPLIT_FP16 ||
-      plan.algo == NUMC_CUDA_ALGO_OZAKI || plan.algo == NUMC_CUDA_ALGO_TC_INT8) {
+      plan.algo == NUMC_CUDA_ALGO_OZAKI || plan.algo == NUMC_CUDA_ALGO_TC_INT8 ||
+      plan.algo == kAlgoIntDigits) {
     unsigned st = 0;
     CU(numc_k::read_and_clear_status(&st, s), "status read");
     if (st) return NUMC_SET_ERROR(NUMC_ERR_INTERNAL, "matmul kernel abandoned a bounded wait (code %u)", st);
@@ -891,9 +935,10 @@ int bmm_impl(const NumcArray *a, const NumcArray *b, NumcArray *out) {
   const size_t off_b = align_up(ra ? 0 : sa, 256);
   const size_t off_o = off_b + align_up(rb ? 0 : sb, 256);
   const size_t off_w = off_o + align_up(ro ? 0 : so, 256);
-  const size_t ws_bytes = plan_workspace(plan, M, K, N);
+  size_t ws_bytes = 0;
   char *scratch = nullptr;
-  if ((err = ctx_scratch(ctx, off_w + ws_bytes + 256, s, &scratch))) return err;
+  if ((err = plan_scratch(ctx, dt, &plan, M, K, N, off_w, ra && rb && ro, s, &ws_bytes,
+                          &scratch))) return err;
   const char *da = ra ? a->dev_base : scratch;
   const char *db = rb ? b->dev_base : scratch + off_b;
   char *dout = ro ? out->dev_base : scratch + off_o;
@@ -1030,7 +1075,6 @@ int dot_impl(const NumcArray *a, const NumcArray *b, NumcArray *out) {
     gemm_branch = P == 1 && csb == 1 && cso == 1;
     if (gemm_branch) {
       if ((err = resolve(dt, NUMC_CUDA_ALGO_DEFAULT, -1, M, K, N, &plan, true))) return err;
-      ws_bytes = plan_workspace(plan, M, K, N);
     }
   } else if (kind == kVector) {
     ws_bytes = numc_k::dot1d_scratch_bytes();
@@ -1045,7 +1089,10 @@ int dot_impl(const NumcArray *a, const NumcArray *b, NumcArray *out) {
   const size_t off_o = off_b + align_up(rb ? 0 : sb, 256);
   const size_t off_w = off_o + align_up(ro ? 0 : so, 256);
   char *scratch = nullptr;
-  if ((err = ctx_scratch(ctx, off_w + ws_bytes + 256, s, &scratch))) return err;
+  if (gemm_branch) err = plan_scratch(ctx, dt, &plan, M, K, N, off_w, ra && rb && ro, s, &ws_bytes,
+                          &scratch);
+  else err = ctx_scratch(ctx, off_w + ws_bytes + 256, s, &scratch);
+  if (err) return err;
   const char *da = ra ? a->dev_base : scratch;
   const char *db = rb ? b->dev_base : scratch + off_b;
   char *dout = ro ? out->dev_base : scratch + off_o;
@@ -1406,7 +1453,7 @@ extern "C" size_t numc_cuda_gemm_workspace_size(NumcDType dt, int algo, int para
   if ((int)dt < 0 || (int)dt >= NUMC_DTYPE_COUNT) return 0;
   Plan p;
   if (resolve(dt, algo, param, M, K, N, &p)) return 0;
-  return plan_workspace(p, M, K, N);
+  return plan_workspace(dt, p, M, K, N);
 }
 
 extern "C" int numc_cuda_gemm(NumcDType dt, int algo, int param, const void *a,
@@ -1427,7 +1474,14 @@ extern "C" int numc_cuda_gemm(NumcDType dt, int algo, int param, const void *a,
   int err = resolve(dt, algo, param, M, K, N, &p);
   if (err) return err;
   cudaStream_t s = (cudaStream_t)stream;
-  size_t need = plan_workspace(p, M, K, N);
+  size_t need = plan_workspace(dt, p, M, K, N);
+  if (p.algo == kAlgoIntDigits &&
+      (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255))) {
+    // The CUDA cores need no workspace: calls without one (or with less)
+    // stay there, and stay independent of each other on any streams.
+    p.algo = NUMC_CUDA_ALGO_SIMT;
+    need = 0;
+  }
   void *ws = workspace;
   size_t ws_bytes = workspace_bytes;
   if (need) {

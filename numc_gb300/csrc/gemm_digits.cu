@@ -122,6 +122,50 @@ __device__ __forceinline__ void load8(const T *row, int64_t rs_k, int64_t k0, in
   }
 }
 
+// The digit pass: a warp takes 8 rows x 32 k (rows of 4 eight-element
+// chunks), a block 64 rows x 32 k.  Contiguous rows are read as whole 128- or
+// 256-byte lines, row-contiguous operands (B, read as B^T) as 8-element
+// segments that fill sectors; per digit a warp writes two runs of 256 bytes.
+// Blocks past both operands' clear C for a K-split GEMM that adds into it.
+template <typename T, int S>
+__global__ void __launch_bounds__(256)
+int_digits(DigitOperand a, DigitOperand b, int64_t K, int64_t Ks, unsigned kgroups,
+           unsigned groups_a, T *zero, int64_t rso, int64_t cso, int64_t M, int64_t N) {
+  if (zero) {
+    const int64_t n = M * N, step = (int64_t)gridDim.x * 256;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += step)
+      zero[i / N * rso + i % N * cso] = 0;
+  }
+  unsigned rg = blockIdx.x / kgroups;
+  const unsigned kg = blockIdx.x % kgroups;
+  const bool second = rg >= groups_a;
+  const DigitOperand &o = second ? b : a;
+  if (second) rg -= groups_a;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t r = (int64_t)rg * 64 + warp * 8 + (lane >> 2);
+  const int64_t k0 = (int64_t)kg * 32 + (lane & 3) * 8;
+  const int kb = (int)(k0 / kKS), c = (int)(k0 / 8) & 1;
+  if (r >= o.R || kb >= Ks) return;
+  T x[8];
+  load8((const T *)o.src + r * o.rs_row, o.rs_k, k0, K, x);
+  // digit + 128 per byte: adding 0x80 to every byte position makes the
+  // bytes of the (wrapped) sum the balanced digits
+  const T c80 = (T)0x8080808080808080ull;
+#pragma unroll
+  for (int i = 0; i < 8; i++) x[i] = (T)(x[i] + c80);
+#pragma unroll
+  for (int p = 0; p < S; p++) {
+    uint32_t h[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint64_t u0 = x[2 * j], u1 = x[2 * j + 1];
+      h[j] = digit_pair((uint32_t)(u0 >> (p & 4) * 8), (uint32_t)(u1 >> (p & 4) * 8), p & 3);
+    }
+    *reinterpret_cast<uint4 *>(o.dst + digit_offset(r, kb, p, c, o.R, o.BR, S, Ks)) =
+        make_uint4(h[0], h[1], h[2], h[3]);
+  }
+}
+
 // ---- float64 ----------------------------------------------------------------
 
 // Bit tests on float64 values: GB300's FP64 pipe is slow, so compares on
@@ -903,6 +947,130 @@ cudaError_t launch_ozaki(const Gemm &g, int slices, void *ws_v, size_t ws_bytes,
   }
   mark.gemm_done();
   return e;
+}
+
+// ---- 16-, 32- and 64-bit integers -------------------------------------------
+
+namespace {
+
+// How an integer problem runs: columns per tile and K splits (0 columns: not
+// here), and the estimated times in us here and on the CUDA cores.
+struct IntPlan {
+  int BN = 0, ksplit = 1;
+  double us = 0, simt_us = 0;
+  int64_t Ks = 0;
+  size_t b = 0, total = 0;
+};
+
+IntPlan int_plan(int bytes, int64_t M, int64_t K, int64_t N) {
+  IntPlan p;
+  if (M <= 0 || N <= 0 || K <= 0 || M >= (1ll << 30) || N >= (1ll << 30) || K >= (1ll << 30))
+    return p;
+  if (!digit_grid(M, K, N).blocks) return p;
+  p.Ks = (K + kKS - 1) / kKS;
+  const int s = bytes, sms = sm_count() > 0 ? sm_count() : 152;
+  double best = 1e30;
+  for (int BN = 64; BN <= 128; BN += 64) {
+    if (bytes == 8 && BN == 128) continue;    // 8 diagonals of 128 columns exceed TMEM
+    const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + BN - 1) / BN);
+    // Measured cycles of a K step (4096^3), of a unit's start and end, and of
+    // adding a tile into C.
+    const double step = bytes == 8 ? 1200 : bytes == 4 ? (BN == 64 ? 424 : 788)
+                                                       : (BN == 64 ? 187 : 275);
+    for (int ks = 1; ks <= 32 && ks <= std::max<int64_t>(1, p.Ks / 4); ks++) {
+      if (ks > 1 && bytes == 2) break;        // no 16-bit atomics
+      const int64_t rounds = (tiles * ks + sms - 1) / sms;
+      const double t =
+          rounds * ((p.Ks + ks - 1) / ks * step + 3000 + (ks > 1 ? 0.7 * kBM * BN : 0));
+      if (t < best) {
+        best = t;
+        p.BN = BN;
+        p.ksplit = ks;
+      }
+    }
+  }
+  // The line to the CUDA cores, from both sides' times (digits / CUDA cores, us,
+  // back to back in a graph, GB300):
+  //            64^3      256^3      512^3      1024^3    2048x128x256  64x5000x64
+  //   int16  6.6/3.2   8.1/7.0    9.4/19.6   14/92       7.3/11.6      52/96
+  //   int32  8.1/3.2  10.5/7.0   11.1/19.3   23/96       9.1/11.6      11/95
+  //   int64 12.5/5.0  13.6/13.8  16.8/45.8   60/335     15.5/25.0      19/225
+  // Here: two launches and the passes' bytes besides the units' cycles; there
+  // the longer of the K loop of one thread and of all multiply-adds (a low
+  // estimate: near the line the CUDA cores keep the problem).
+  const double elems = (double)(M + N) * K, out = (double)M * N;
+  p.us = 5.5 + best / 1900 + elems * 3 * bytes / 4e6 + out * bytes * (p.ksplit > 1 ? 2 : 1) / 3e6;
+  p.simt_us = 2.5 + std::max(K * (bytes == 8 ? 0.042 : 0.0185),
+                             2 * out * K / (bytes == 8 ? 6.4e6 : 18e6));
+  p.b = (size_t)round_up((int64_t)s * M * p.Ks * kKS * 2, 256);
+  p.total = p.b + (size_t)round_up((int64_t)s * N * p.Ks * kKS * 2, 256);
+  return p;
+}
+
+int int_bytes(NumcDType dt) {
+  switch (dt) {
+  case NUMC_DTYPE_INT16: case NUMC_DTYPE_UINT16: return 2;
+  case NUMC_DTYPE_INT32: case NUMC_DTYPE_UINT32: return 4;
+  case NUMC_DTYPE_INT64: case NUMC_DTYPE_UINT64: return 8;
+  default: return 0;
+  }
+}
+
+template <typename T>
+cudaError_t run_int(const Gemm &g, const IntPlan &ip, char *ws, unsigned *status,
+                    cudaStream_t s) {
+  constexpr int S = sizeof(T);
+  const DigitGrid dg = digit_grid(g.M, g.K, g.N);
+  const DigitOperand oa{g.a, g.rsa, g.csa, g.M, (uint16_t *)ws, kBM};
+  const DigitOperand ob{g.b, g.csb, g.rsb, g.N, (uint16_t *)(ws + ip.b), ip.BN};
+  PhaseMark mark(s);
+  int_digits<T, S><<<dg.blocks, 256, 0, s>>>(oa, ob, g.K, ip.Ks, dg.kgroups, dg.groups_a,
+                                             ip.ksplit > 1 ? (T *)g.c : nullptr, g.rso, g.cso,
+                                             g.M, g.N);
+  count_launch();
+  cudaError_t e = cudaGetLastError();
+  if (e) return e;
+  mark.split_done();
+  DigitGemm P = {};
+  P.pa = oa.dst;
+  P.pb = ob.dst;
+  P.rso = g.rso; P.cso = g.cso;
+  P.M = (int)g.M; P.N = (int)g.N; P.Ks = (int)ip.Ks;
+  P.ksplit = ip.ksplit;
+  P.status = status;
+  P.bias = g.bias;
+  P.bias_stride = g.bias_stride;
+  if constexpr (S == 8) e = launch_digit_gemm<8, 64, T>(P, (T *)g.c, s);
+  else e = ip.BN == 64 ? launch_digit_gemm<S, 64, T>(P, (T *)g.c, s)
+                       : launch_digit_gemm<S, 128, T>(P, (T *)g.c, s);
+  mark.gemm_done();
+  return e;
+}
+
+}  // namespace
+
+size_t int_digits_workspace(NumcDType dt, int64_t M, int64_t K, int64_t N) {
+  const int bytes = int_bytes(dt);
+  if (!bytes) return 0;
+  const IntPlan p = int_plan(bytes, M, K, N);
+  return p.BN && p.us < p.simt_us ? p.total : 0;
+}
+
+double int_digits_gain_us(NumcDType dt, int64_t M, int64_t K, int64_t N) {
+  const IntPlan p = int_plan(int_bytes(dt), M, K, N);
+  return p.BN ? p.simt_us - p.us : 0;
+}
+
+cudaError_t launch_int_digits(NumcDType dt, const Gemm &g, void *ws, size_t ws_bytes,
+                              cudaStream_t s) {
+  const int bytes = int_bytes(dt);
+  const IntPlan p = int_plan(bytes, g.M, g.K, g.N);
+  if (!bytes || !p.BN || ws_bytes < p.total || ((uintptr_t)ws & 255)) return cudaErrorInvalidValue;
+  unsigned *status = status_word();
+  if (!status) return cudaErrorMemoryAllocation;
+  if (bytes == 8) return run_int<unsigned long long>(g, p, (char *)ws, status, s);
+  if (bytes == 4) return run_int<unsigned>(g, p, (char *)ws, status, s);
+  return run_int<unsigned short>(g, p, (char *)ws, status, s);
 }
 
 }  // namespace numc_k
