@@ -111,12 +111,18 @@ cudaError_t launch_sized(const Gemm &g, int rule8, cudaStream_t s) {
   return launch_tile<T, 32, 32, 2, 2, KIND, 32>(g, rule8, s);
 }
 
-// numc's packed float path: 64- and 32-wide tiles sum the remainder-tile
+// numc's packed float path.  float32 takes the packed-FMA kernel; what that
+// leaves (problems of few tiles, huge strides) and float64 run here: 64- and
+// 32-wide tiles sum the remainder-tile
 // outputs per K block in the tile kernel (kFloatEdges); 128-wide tiles
 // (8 x 8 outputs a thread, no registers to spare) leave them to the
 // float_edges pass.
 template <typename T, int BIG>
 cudaError_t launch_float_packed(const Gemm &g, cudaStream_t s) {
+  if constexpr (std::is_same<T, float>::value) {
+    cudaError_t e = cudaSuccess;
+    if (g.M > 0 && g.N > 0 && g.K > 0 && launch_f32_packed(g, s, &e)) return e;
+  }
   int t = BIG;
   while (t > 32 && ((g.M + t - 1) / t) * ((g.N + t - 1) / t) < sms()) t /= 2;
   cudaError_t e;
