@@ -111,9 +111,9 @@ cudaError_t launch_sized(const Gemm &g, int rule8, cudaStream_t s) {
   return launch_tile<T, 32, 32, 2, 2, KIND, 32>(g, rule8, s);
 }
 
-// numc's packed float path.  float32 takes the packed-FMA kernel; what that
-// leaves (problems of few tiles, huge strides) and float64 run here: 64- and
-// 32-wide tiles sum the remainder-tile
+// numc's packed float path.  float32 takes the kernels of gemm_f32.cu unless
+// its strides are huge; float64 (and that rest) runs here: 64- and 32-wide
+// tiles sum the remainder-tile
 // outputs per K block in the tile kernel (kFloatEdges); 128-wide tiles
 // (8 x 8 outputs a thread, no registers to spare) leave them to the
 // float_edges pass.
@@ -159,7 +159,11 @@ cudaError_t launch_simt(NumcDType dt, const Gemm &g_in, int rule8, cudaStream_t 
   case NUMC_DTYPE_FLOAT32:
     switch (rule8) {
     case kFloatNaive: return launch_sized<float, simt::kFloatUnfused, 128>(g, 0, s);
-    case kFloatNumcSmall: return launch_sized<float, simt::kFloatSmall, 128>(g, 0, s);
+    case kFloatNumcSmall: {
+      cudaError_t e = cudaSuccess;
+      if (g.M > 0 && g.N > 0 && g.K > 0 && launch_f32_unpacked(g, s, &e)) return e;
+      return launch_sized<float, simt::kFloatSmall, 128>(g, 0, s);
+    }
     default: return launch_float_packed<float, 128>(g, s);
     }
   case NUMC_DTYPE_FLOAT64:

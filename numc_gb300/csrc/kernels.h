@@ -62,9 +62,11 @@ enum FloatSimt : int {
 // CUDA-core kernels for every dtype.  `rule8` is the Rule8 for int8/uint8,
 // the FloatSimt variant for float32/float64, unused otherwise.
 cudaError_t launch_simt(NumcDType dt, const Gemm &g, int rule8, cudaStream_t s);
-// float32, numc's packed-path arithmetic, with packed FMAs: false where the
-// problem is too small for its tiles (or its strides too large).
+// float32, numc's packed-path arithmetic (gemm_f32.cu): false where the strides
+// or K exceed its 32-bit offsets.
 bool launch_f32_packed(const Gemm &g, cudaStream_t s, cudaError_t *e);
+// The same for numc's unpacked path.
+bool launch_f32_unpacked(const Gemm &g, cudaStream_t s, cudaError_t *e);
 // The float variant kFloatNumc resolves to for problem g.
 int float_rule(NumcDType dt, const Gemm &g, int rule);
 // The float tile geometry (NumcIsa) of the process-wide ISA profile.

@@ -84,3 +84,24 @@ def test_linear_bias_and_special_values():
     np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
     ok = ~np.isnan(want)
     assert got[ok].tobytes() == want[ok].tobytes()
+
+
+# small tiles (16 x 16 and 32 x 32, packed and unpacked path): tile edges, K
+# around the slabs of 32 and 64, operands that 16-byte copies take and others
+SMALL = [(1, 1, 1), (16, 64, 16), (17, 65, 15), (96, 96, 96), (95, 97, 96), (10, 1000, 80),
+         (256, 128, 10), (64, 256, 64), (64, 257, 64), (100, 1024, 33), (256, 784, 128),
+         (130, 600, 260), (512, 300, 512), (511, 301, 513), (2, 3000, 1000)]
+
+
+@pytest.mark.parametrize("profile", [nc.INT8_X86_AVX2, nc.INT8_ARM_NEON], ids=["x86", "neon"])
+@pytest.mark.parametrize("shape", SMALL, ids=lambda s: "x".join(map(str, s)))
+def test_small_tiles_bit_identical(shape, profile):
+    M, K, N = shape
+    a, b = synth.operands("uniform", M, K, N, seed=6)
+    want = oracle.matmul(a, b, profile).tobytes()
+    ta, tb = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    at, bt = ta.t().contiguous().t(), tb.t().contiguous().t()
+    wide = torch.zeros((M, K + 1), device="cuda")
+    wide[:, 1:] = ta
+    for x, y in ((ta, tb), (at, bt), (ta, bt), (wide[:, 1:], tb)):
+        assert _run(x, y, profile).tobytes() == want
