@@ -335,38 +335,9 @@ __device__ __forceinline__ void load_planes(uint32_t dst, const uint16_t *src, i
   }
 }
 
-// One lane of a converged warp.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t ok;
-  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
-               : "=r"(ok));
-  return ok != 0;
-}
-
-// tcgen05.mma / commit by the elected lane of a converged warp, predicated
-// rather than branched around.
-__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
-                                        uint32_t accumulate, bool lead) {
-  asm volatile(
-      "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
-      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"((uint32_t)lead)
-      : "memory");
-}
-__device__ __forceinline__ void commit(uint64_t *bar, bool lead) {
-  asm volatile(
-      "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
-      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(
-          tc::smem_u32(bar)),
-      "r"((uint32_t)lead)
-      : "memory");
-}
-
-// Bounded wait by a whole warp; all lanes agree on the outcome.
 __device__ __forceinline__ bool wait_all(uint64_t *bar, uint32_t parity, const DigitGemm &P,
                                          unsigned code = kStatusTimeoutMma) {
-  return __all_sync(0xffffffffu, tc::mbar_wait_bounded(tc::smem_u32(bar), parity, P.status, code,
-                                                       P.wc.limit_ns));
+  return tc::mbar_wait_warp(tc::smem_u32(bar), parity, P.status, code, P.wc.limit_ns);
 }
 
 // (hi, frac) += t, a signed 64-bit number in units of the fraction.
@@ -514,7 +485,7 @@ __device__ __forceinline__ void issue_group(const DigitGemm &P, uint8_t *smem, u
   using Cfg = DigitCfg<S, BN, T>;
   constexpr int NS = Cfg::NS, ST = Cfg::STAGES, NBUF = Cfg::NBUF;
   constexpr uint32_t A_PLANE = kBM * kRowBytes / 16, B_PLANE = BN * kRowBytes / 16;
-  const bool lead = elect_one();
+  const bool lead = tc::elect_one();
   const int units = P.tiles_m * P.tiles_n * P.ksplit;
   int g = 0, chunk = 0;   // stages and chunks across units
   for (int u = blockIdx.x; u < units; u += gridDim.x) {
@@ -542,14 +513,14 @@ __device__ __forceinline__ void issue_group(const DigitGemm &P, uint8_t *smem, u
 #pragma unroll
             for (int d = p > D0 ? p : D0; d < D1; d += W) {
               const int n = D1 - d < W ? D1 - d : W;
-              mma_f16(d0 + d * BN, sdesc(sa + p * A_PLANE), sdesc(sb + (d - p) * B_PLANE),
+              tc::mma_f16_lead(d0 + d * BN, sdesc(sa + p * A_PLANE), sdesc(sb + (d - p) * B_PLANE),
                       tc::idesc_f16_f32(kBM, n * BN), p > 0 ? 1u : ks + i > kc, lead);
             }
           }
         }
-        commit(&empty[st], lead);
+        tc::mma_commit_lead(tc::smem_u32(&empty[st]), lead);
       }
-      commit(&tfull[2 * buf + GROUP], lead);
+      tc::mma_commit_lead(tc::smem_u32(&tfull[2 * buf + GROUP]), lead);
     }
   }
 }
@@ -630,7 +601,7 @@ digit_gemm(const DigitGemm P, T *__restrict__ C) {
     // Every MMA issued above completes before TMEM is released, also when
     // the loop gave up (a commit with none outstanding arrives at once).
     if (warp == 1 || S > LOW) {
-      commit(drain, elect_one());
+      tc::mma_commit_lead(tc::smem_u32(drain), tc::elect_one());
       wait_all(drain, 0, P, kStatusTimeoutDrain);
     }
   } else {

@@ -235,24 +235,28 @@ grouped_split_gemm(const CUtensorMap *__restrict__ tmaps, const Prob *__restrict
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool lead = tc::elect_one();
       constexpr uint32_t idesc = F16 ? tc::idesc_f16_f32(kBM, BN) : tc::idesc_bf16_f32(kBM, BN);
       int g = 0, chunk = 0;
       bool live = true;
       for (int t = blockIdx.x; t < ntiles && live; t += gridDim.x) {
         int kb0, kb1;
         slice_range(probs[tiles[t].prob], tiles[t].ks, kb0, kb1);
+        // loaded values made uniform for the compiler too
+        kb1 = (int)__reduce_max_sync(0xffffffffu, (unsigned)(kb1 - kb0));
+        kb0 = 0;
         for (int kb = kb0; kb < kb1; kb++, g++) {
           const int s = g % STAGES, buf = chunk % NBUF;
           const bool cstart = (kb - kb0) % FLUSH == 0;
           const bool cend = (kb - kb0) % FLUSH == FLUSH - 1 || kb == kb1 - 1;
           if (cstart && chunk >= NBUF &&
-              !tc::mbar_wait_bounded(tc::smem_u32(&tempty[buf]), ((chunk / NBUF) & 1) ^ 1,
+              !tc::mbar_wait_warp(tc::smem_u32(&tempty[buf]), ((chunk / NBUF) & 1) ^ 1,
                                      status, kStatusTimeoutMma, wc.limit_ns)) {
             live = false;
             break;
           }
-          if (!tc::mbar_wait_bounded(tc::smem_u32(&full[s]), (g / STAGES) & 1, status,
+          if (!tc::mbar_wait_warp(tc::smem_u32(&full[s]), (g / STAGES) & 1, status,
                                      kStatusTimeoutMma, wc.limit_ns)) {
             live = false;
             break;
@@ -266,25 +270,24 @@ grouped_split_gemm(const CUtensorMap *__restrict__ tmaps, const Prob *__restrict
           const uint32_t d = tmem + buf * BN;
 #pragma unroll
           for (int kk = 0; kk < kBK / 16; kk++)
-            tc::mma_bf16(d, tc::sdesc_k128(a1 + kk * 32), tc::sdesc_k128(b0 + kk * 32), idesc,
-                         (!cstart || kk > 0) ? 1u : 0u);
+            tc::mma_f16_lead(d, tc::sdesc_k128(a1 + kk * 32), tc::sdesc_k128(b0 + kk * 32), idesc, (!cstart || kk > 0) ? 1u : 0u, lead);
 #pragma unroll
           for (int kk = 0; kk < kBK / 16; kk++)
-            tc::mma_bf16(d, tc::sdesc_k128(a0 + kk * 32), tc::sdesc_k128(b1 + kk * 32), idesc, 1u);
+            tc::mma_f16_lead(d, tc::sdesc_k128(a0 + kk * 32), tc::sdesc_k128(b1 + kk * 32), idesc, 1u, lead);
 #pragma unroll
           for (int kk = 0; kk < kBK / 16; kk++)
-            tc::mma_bf16(d, tc::sdesc_k128(a0 + kk * 32), tc::sdesc_k128(b0 + kk * 32), idesc, 1u);
-          tc::mma_commit(tc::smem_u32(&empty[s]));
+            tc::mma_f16_lead(d, tc::sdesc_k128(a0 + kk * 32), tc::sdesc_k128(b0 + kk * 32), idesc, 1u, lead);
+          tc::mma_commit_lead(tc::smem_u32(&empty[s]), lead);
           if (cend) {
-            tc::mma_commit(tc::smem_u32(&tfull[buf]));
+            tc::mma_commit_lead(tc::smem_u32(&tfull[buf]), lead);
             chunk++;
           }
         }
       }
       // Every MMA issued above completes before TMEM is released, also when
       // the loop gave up (a commit with none outstanding arrives at once).
-      tc::mma_commit(tc::smem_u32(drain));
-      tc::mbar_wait_bounded(tc::smem_u32(drain), 0, status, kStatusTimeoutDrain, wc.limit_ns);
+      tc::mma_commit_lead(tc::smem_u32(drain), lead);
+      tc::mbar_wait_warp(tc::smem_u32(drain), 0, status, kStatusTimeoutDrain, wc.limit_ns);
     }
     __syncwarp();
   } else {

@@ -321,31 +321,33 @@ int8_tc_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUt
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool lead = tc::elect_one();
       constexpr uint32_t idesc = tc::idesc_bf16_f32(kBM, kBN);
       for (int kb = 0; kb < num_kb; kb++) {
         const int s = kb % kStages, chunk = kb >> chunk_log2, buf = chunk % kNumBuf;
         const bool cstart = (kb & (CHUNK - 1)) == 0, cend = (kb & (CHUNK - 1)) == CHUNK - 1;
         if (cstart && chunk >= kNumBuf &&
-            !tc::mbar_wait_bounded(tc::smem_u32(&tempty[buf]), ((chunk / kNumBuf) & 1) ^ 1,
+            !tc::mbar_wait_warp(tc::smem_u32(&tempty[buf]), ((chunk / kNumBuf) & 1) ^ 1,
                                    status, kStatusTimeoutMma, wc.limit_ns))
           break;
-        if (!tc::mbar_wait_bounded(tc::smem_u32(&full[s]), (kb / kStages) & 1, status,
+        if (!tc::mbar_wait_warp(tc::smem_u32(&full[s]), (kb / kStages) & 1, status,
                                    kStatusTimeoutMma, wc.limit_ns))
           break;
         tc::tc_fence_after();
         const uint32_t sa = tc::smem_u32(smem + s * STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
         for (int kk = 0; kk < kBK / 16; kk++)
-          tc::mma_bf16(tmem + buf * kBN, tc::sdesc_k128(sa + kk * 32),
-                       tc::sdesc_k128(sb + kk * 32), idesc, (!cstart || kk > 0) ? 1u : 0u);
-        tc::mma_commit(tc::smem_u32(&empty[s]));
-        if (cend) tc::mma_commit(tc::smem_u32(&tfull[buf]));
+          tc::mma_f16_lead(tmem + buf * kBN, tc::sdesc_k128(sa + kk * 32),
+                           tc::sdesc_k128(sb + kk * 32), idesc, (!cstart || kk > 0) ? 1u : 0u,
+                           lead);
+        tc::mma_commit_lead(tc::smem_u32(&empty[s]), lead);
+        if (cend) tc::mma_commit_lead(tc::smem_u32(&tfull[buf]), lead);
       }
       // Every MMA issued above completes before TMEM is released, also when
       // the loop gave up (a commit with none outstanding arrives at once).
-      tc::mma_commit(tc::smem_u32(drain));
-      tc::mbar_wait_bounded(tc::smem_u32(drain), 0, status, kStatusTimeoutDrain, wc.limit_ns);
+      tc::mma_commit_lead(tc::smem_u32(drain), lead);
+      tc::mbar_wait_warp(tc::smem_u32(drain), 0, status, kStatusTimeoutDrain, wc.limit_ns);
     }
     __syncwarp();
   } else {
@@ -601,7 +603,8 @@ int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool lead = tc::elect_one();
       constexpr uint32_t idesc = tc::idesc_bf16_f32(2 * kBM, BN);
       int g = 0, chunk = 0;   // stage and chunk counters across tiles
       bool live = true;
@@ -611,12 +614,12 @@ int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
           const bool cstart = kb % CHUNK == 0;
           const bool cend = kb % CHUNK == CHUNK - 1 || kb == num_kb - 1;
           if (cstart && chunk >= NBUF &&
-              !tc::mbar_wait_bounded(tc::smem_u32(&tempty[buf]), ((chunk / NBUF) & 1) ^ 1,
+              !tc::mbar_wait_warp(tc::smem_u32(&tempty[buf]), ((chunk / NBUF) & 1) ^ 1,
                                      status, kStatusTimeoutMma, wc.limit_ns)) {
             live = false;
             break;
           }
-          if (!tc::mbar_wait_bounded(tc::smem_u32(&full[s]), (g / STAGES) & 1, status,
+          if (!tc::mbar_wait_warp(tc::smem_u32(&full[s]), (g / STAGES) & 1, status,
                                      kStatusTimeoutMma, wc.limit_ns)) {
             live = false;
             break;
@@ -625,19 +628,20 @@ int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
           const uint32_t sa = tc::smem_u32(smem + s * Cfg::STAGE_BYTES), sb = sa + Cfg::A_BYTES;
 #pragma unroll
           for (int kk = 0; kk < kBK / 16; kk++)
-            tc::mma_f16_pair(tmem + buf * BN, tc::sdesc_k128(sa + kk * 32),
-                             tc::sdesc_k128(sb + kk * 32), idesc, (!cstart || kk > 0) ? 1u : 0u);
-          tc::mma_commit_pair(tc::smem_u32(&empty[s]), 0x3);
+            tc::mma_f16_lead<2>(tmem + buf * BN, tc::sdesc_k128(sa + kk * 32),
+                                tc::sdesc_k128(sb + kk * 32), idesc,
+                                (!cstart || kk > 0) ? 1u : 0u, lead);
+          tc::mma_commit_lead<2>(tc::smem_u32(&empty[s]), lead);
           if (cend) {
-            tc::mma_commit_pair(tc::smem_u32(&tfull[buf]), 0x3);
+            tc::mma_commit_lead<2>(tc::smem_u32(&tfull[buf]), lead);
             chunk++;
           }
         }
       }
       // Every MMA issued above completes before TMEM is released, also when
       // the loop gave up (a commit with none outstanding arrives at once).
-      tc::mma_commit_pair(tc::smem_u32(drain), 0x1);
-      tc::mbar_wait_bounded(tc::smem_u32(drain), 0, status, kStatusTimeoutDrain, wc.limit_ns);
+      tc::mma_commit_lead<2>(tc::smem_u32(drain), lead, 0x1);
+      tc::mbar_wait_warp(tc::smem_u32(drain), 0, status, kStatusTimeoutDrain, wc.limit_ns);
     }
     __syncwarp();
   } else {

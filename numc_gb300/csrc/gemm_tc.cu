@@ -400,7 +400,7 @@ template <> struct Products<3> {
 
 // Warp roles (64 + 32 * BN / 16 threads per CTA):
 //   warp 0, lane 0   TMA producer: fills the STAGES-deep ring of K slabs.
-//   warp 1, lane 0   MMA issuer: for chunk c (FLUSH consecutive K slabs),
+//   warp 1           MMA issuer: for chunk c (FLUSH consecutive K slabs),
 //                    accumulates all products into TMEM buffer c % NBUF
 //                    (starting from zero) and commits it to the
 //                    accumulator warps.
@@ -531,7 +531,8 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool lead = tc::elect_one();
       constexpr uint32_t idesc =
           F16 ? tc::idesc_f16_f32(kBM * CTAS, BN) : tc::idesc_bf16_f32(kBM * CTAS, BN);
       int g = 0, chunk = 0;   // stage and chunk counters across tiles
@@ -542,12 +543,12 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
           const bool chunk_start = kb % FLUSH == 0;
           const bool chunk_end = kb % FLUSH == FLUSH - 1 || kb == num_kb - 1;
           if (chunk_start && chunk >= NBUF &&
-              !tc::mbar_wait_bounded(tc::smem_u32(&tempty[buf]), ((chunk / NBUF) & 1) ^ 1,
+              !tc::mbar_wait_warp(tc::smem_u32(&tempty[buf]), ((chunk / NBUF) & 1) ^ 1,
                                      status, kStatusTimeoutMma, wc.limit_ns)) {
             live = false;
             break;
           }
-          if (!tc::mbar_wait_bounded(tc::smem_u32(&full[s]), (g / STAGES) & 1, status,
+          if (!tc::mbar_wait_warp(tc::smem_u32(&full[s]), (g / STAGES) & 1, status,
                                      kStatusTimeoutMma, wc.limit_ns)) {
             live = false;
             break;
@@ -568,26 +569,19 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
               const uint32_t acc = (!chunk_start || kk > 0 || p > 0) ? 1u : 0u;
               const uint64_t ad = tc::sdesc_k128(st + P::a(p) * Cfg::A_BYTES + koff);
               const uint64_t bd = tc::sdesc_k128(bbase + P::b(p) * Cfg::B_BYTES + koff);
-              if constexpr (PAIR) tc::mma_f16_pair(acc_tmem, ad, bd, idesc, acc);
-              else tc::mma_bf16(acc_tmem, ad, bd, idesc, acc);
+              tc::mma_f16_lead<CTAS>(acc_tmem, ad, bd, idesc, acc, lead);
             }
           }
-          if constexpr (PAIR) {
-            tc::mma_commit_pair(tc::smem_u32(&empty[s]), 0x3);
-            if (chunk_end) tc::mma_commit_pair(tc::smem_u32(&tfull[buf]), 0x3);
-          } else {
-            tc::mma_commit(tc::smem_u32(&empty[s]));
-            if (chunk_end) tc::mma_commit(tc::smem_u32(&tfull[buf]));
-          }
+          tc::mma_commit_lead<CTAS>(tc::smem_u32(&empty[s]), lead);
+          if (chunk_end) tc::mma_commit_lead<CTAS>(tc::smem_u32(&tfull[buf]), lead);
           if (chunk_end) chunk++;
         }
       }
       // Whether the loop ran to the end or gave up, every MMA issued above
       // completes before TMEM is released (a commit with none outstanding
       // arrives at once).
-      if constexpr (PAIR) tc::mma_commit_pair(tc::smem_u32(drain), 0x1);
-      else tc::mma_commit(tc::smem_u32(drain));
-      tc::mbar_wait_bounded(tc::smem_u32(drain), 0, status, kStatusTimeoutDrain, wc.limit_ns);
+      tc::mma_commit_lead<CTAS>(tc::smem_u32(drain), lead, 0x1);
+      tc::mbar_wait_warp(tc::smem_u32(drain), 0, status, kStatusTimeoutDrain, wc.limit_ns);
     }
     __syncwarp();
   } else {

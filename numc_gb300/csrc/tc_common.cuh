@@ -180,24 +180,6 @@ __host__ __device__ constexpr uint32_t idesc_f16_f32(int M, int N) {
   return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by a single thread.
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Arrive once on `bar` when all previously issued tcgen05.mma of this
-// thread have completed.
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-      : "memory");
-}
-
 // 32 lanes x 32 bits, 32 consecutive columns: thread t of the warp gets
 // row (lane base + t), columns [col, col + 32).
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -259,6 +241,67 @@ __device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t
 
 __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// ---- Issue by a whole warp -----------------------------------------------------
+//
+// A loop of one lane that builds descriptors and issues MMAs moves every
+// operand into uniform registers one MMA at a time: some 100 cycles an MMA,
+// more than MMAs of up to 128 columns take.  With the whole warp in the loop
+// and the instruction predicated on an elected lane the operands stay in
+// uniform registers.
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(ok));
+  return ok != 0;
+}
+
+// D (+)= A B^T, kind::f16 (operand types in idesc), by the lane with `lead`;
+// CTAS = 2: on a CTA pair, called by the even CTA's warp.
+template <int CTAS = 1>
+__device__ __forceinline__ void mma_f16_lead(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                             uint32_t accumulate, bool lead) {
+  if constexpr (CTAS == 1)
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"((uint32_t)lead)
+        : "memory");
+  else
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+        " @q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"((uint32_t)lead)
+        : "memory");
+}
+
+// Arrive once on `bar` (CTAS = 2: of the CTAs in `mask`) when the leading
+// lane's earlier MMAs have completed.
+template <int CTAS = 1>
+__device__ __forceinline__ void mma_commit_lead(uint32_t bar, bool lead, uint16_t mask = 0x3) {
+  if constexpr (CTAS == 1)
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(
+            bar),
+        "r"((uint32_t)lead)
+        : "memory");
+  else
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+        " @q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
+        " [%0], %2;\n}\n" ::"r"(bar),
+        "r"((uint32_t)lead), "h"(mask)
+        : "memory");
+}
+
+// Bounded wait by a whole warp; all lanes agree on the outcome.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, unsigned *status,
+                                               unsigned code, uint64_t limit_ns) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, status, code, limit_ns));
 }
 
 // ---- CTA pairs: clusters of two CTAs sharing one tcgen05 MMA ------------------
@@ -346,27 +389,6 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncol
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                : "memory");
-}
-
-// D[tmem of both CTAs] (+)= A[smem of both] * B[smem of both]^T; issued by
-// one thread of the even CTA.
-__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                             uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Arrive once on the mbarrier at shared::cta offset `bar` of every CTA in
-// `cta_mask` when all earlier tcgen05.mma of this thread have completed.
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint16_t cta_mask) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
-      " [%0], %1;" ::"r"(bar),
-      "h"(cta_mask)
-      : "memory");
 }
 
 }  // namespace tc
