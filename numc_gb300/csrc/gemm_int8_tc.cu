@@ -520,7 +520,7 @@ template <bool SIGNED, int BN, bool X86>
 __global__ void __launch_bounds__(I8PairCfg<BN>::THREADS, 1)
 int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB,
                uint8_t *__restrict__ C, int64_t rso, int64_t cso, int M, int N, int num_kb,
-               int tiles_m, int tiles_n, int rule, unsigned *status, WaitCfg wc) {
+               int tiles_m, int tiles_n, int bn, int rule, unsigned *status, WaitCfg wc) {
   using Cfg = I8PairCfg<BN>;
   constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, CW = Cfg::CW;
   // slabs per TMEM chunk: the x86 rule folds every 512-deep block; the
@@ -546,7 +546,7 @@ int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
     const int gm = min(tiles_m - first_m, GM);
     const int local = t - group * GM * tiles_n;
     m0 = (first_m + local % gm) * (2 * kBM);
-    n0 = (local / gm) * BN;
+    n0 = (local / gm) * bn;
   };
 
   if (threadIdx.x == 0) {
@@ -581,7 +581,7 @@ int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
       for (int t = first_tile; t < ntiles && live; t += tile_step) {
         int m0, n0;
         tile_origin(t, m0, n0);
-        const int ma = m0 + (int)rank * kBM, nb = n0 + (int)rank * Cfg::BN_CTA;
+        const int ma = m0 + (int)rank * kBM, nb = n0 + (int)rank * (bn / 2);
         for (int kb = 0; kb < num_kb; kb++, g++) {
           const int s = g % STAGES;
           if (g >= STAGES &&
@@ -594,7 +594,7 @@ int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
           const uint32_t fbar = tc::smem_u32(&full[s]);
           const uint32_t st = tc::smem_u32(smem + s * Cfg::STAGE_BYTES);
           // the even CTA's full barrier counts the bytes of both CTAs
-          if (leader) tc::mbar_arrive_expect_tx(fbar, 2 * Cfg::STAGE_BYTES);
+          if (leader) tc::mbar_arrive_expect_tx(fbar, 2 * Cfg::A_BYTES + (uint32_t)bn * kBK * 2);
           const uint32_t fbar_leader = tc::mapa_shared(fbar, 0);
           tc::tma_load_3d_pair(st, &tA, fbar_leader, kb * kBK, ma, 0);
           tc::tma_load_3d_pair(st + Cfg::A_BYTES, &tB, fbar_leader, kb * kBK, nb, 0);
@@ -605,7 +605,7 @@ int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
   } else if (warp == 1) {
     if (leader) {
       const bool lead = tc::elect_one();
-      constexpr uint32_t idesc = tc::idesc_bf16_f32(2 * kBM, BN);
+      const uint32_t idesc = tc::idesc_bf16_f32(2 * kBM, 0) | (uint32_t)(bn >> 3) << 17;
       int g = 0, chunk = 0;   // stage and chunk counters across tiles
       bool live = true;
       for (int t = first_tile; t < ntiles && live; t += tile_step) {
@@ -744,6 +744,7 @@ int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
           tc::mbar_arrive_cluster_relaxed(tc::mapa_shared(tc::smem_u32(&tempty[buf]), 0));
       }
       if (!ok) break;
+      const int Nt = min(N, n0 + bn);   // the tile's columns end here
       uint32_t w[CW / 4];
       if constexpr (X86) {
 #pragma unroll
@@ -765,11 +766,11 @@ int8_pair_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ C
         pack_bytes<CW>(d, w);
       }
       if (staged) {   // warp-uniform
-        store_bytes_coalesced<CW>(w, stage, C, rso, mr + quad * 32, n0 + cbase, M, N, lane);
+        store_bytes_coalesced<CW>(w, stage, C, rso, mr + quad * 32, n0 + cbase, M, Nt, lane);
       } else if (row < M) {
 #pragma unroll
         for (int j = 0; j < CW; j++)
-          if (n0 + cbase + j < N)
+          if (n0 + cbase + j < Nt)
             C[(int64_t)row * rso + (int64_t)(n0 + cbase + j) * cso] = (uint8_t)(w[j >> 2] >> (8 * (j & 3)));
       }
       __syncwarp();   // reconverge before the next tile's tcgen05.ld
@@ -839,21 +840,21 @@ cudaError_t launch_i8_gemm(const Gemm &g, int rule, const I8Layout &L, __nv_bflo
 
 template <bool SIGNED, int BN, bool X86>
 cudaError_t launch_i8_pair(const Gemm &g, int rule, const I8Layout &L, const __nv_bfloat16 *pa,
-                           const __nv_bfloat16 *pb, unsigned *status, cudaStream_t s) {
+                           const __nv_bfloat16 *pb, int bn, unsigned *status, cudaStream_t s) {
   using Cfg = I8PairCfg<BN>;
   CUtensorMap ta, tb;
   cudaError_t e;
   if ((e = make_tmap_3d(&ta, pa, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 1, g.M, L.Kp, L.Kp, kBM,
                         kBK)))
     return e;
-  if ((e = make_tmap_3d(&tb, pb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 1, g.N, L.Kp, L.Kp,
-                        Cfg::BN_CTA, kBK)))
+  if ((e = make_tmap_3d(&tb, pb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 1, g.N, L.Kp, L.Kp, bn / 2,
+                        kBK)))
     return e;
   auto kern = int8_pair_gemm<SIGNED, BN, X86>;
   static LaunchCache lc;
   if ((e = smem_attr_once(lc, (const void *)kern, Cfg::SMEM))) return e;
   const int tiles_m = (int)((g.M + 2 * kBM - 1) / (2 * kBM));
-  const int tiles_n = (int)((g.N + BN - 1) / BN);
+  const int tiles_n = (int)((g.N + bn - 1) / bn);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -875,7 +876,7 @@ cudaError_t launch_i8_pair(const Gemm &g, int rule, const I8Layout &L, const __n
   cfg.gridDim = dim3((unsigned)(2 * pairs));
   cfg.numAttrs = 2;
   e = cudaLaunchKernelEx(&cfg, kern, ta, tb, (uint8_t *)g.c, (int64_t)g.rso, (int64_t)g.cso,
-                         (int)g.M, (int)g.N, (int)(L.Kp / kBK), tiles_m, tiles_n, rule, status,
+                         (int)g.M, (int)g.N, (int)(L.Kp / kBK), tiles_m, tiles_n, bn, rule, status,
                          wait_cfg());
   if (e != cudaSuccess) return e;
   count_launch();
@@ -920,13 +921,19 @@ cudaError_t launch_i8(const Gemm &g, int rule, int tile, char *ws, const I8Layou
   if (e) return e;
   mark.split_done();
   const bool x86 = rule == kRuleX86Packed;
-  if (tile == kI8TileAuto) tile = pick_tile(g);
+  // auto: the pairs' tiles a little narrower than 256 columns where those
+  // round better over the device (4096^2: 224 columns, GEMM 86 -> 83 us)
+  int bn = tile == kI8TilePair128 ? 128 : 256;
+  if (tile == kI8TileAuto) {
+    tile = pick_tile(g);
+    bn = pair_tile_columns(g.M, g.N);
+  }
   if (tile == kI8TilePair256)
-    e = x86 ? launch_i8_pair<SIGNED, 256, true>(g, rule, L, pa, pb, status, s)
-            : launch_i8_pair<SIGNED, 256, false>(g, rule, L, pa, pb, status, s);
+    e = x86 ? launch_i8_pair<SIGNED, 256, true>(g, rule, L, pa, pb, bn, status, s)
+            : launch_i8_pair<SIGNED, 256, false>(g, rule, L, pa, pb, bn, status, s);
   else if (tile == kI8TilePair128)
-    e = x86 ? launch_i8_pair<SIGNED, 128, true>(g, rule, L, pa, pb, status, s)
-            : launch_i8_pair<SIGNED, 128, false>(g, rule, L, pa, pb, status, s);
+    e = x86 ? launch_i8_pair<SIGNED, 128, true>(g, rule, L, pa, pb, bn, status, s)
+            : launch_i8_pair<SIGNED, 128, false>(g, rule, L, pa, pb, bn, status, s);
   else if (((g.M + kBM - 1) / kBM) * ((g.N + 127) / 128) >= sm_count())
     e = launch_i8_gemm<SIGNED, 128>(g, rule, L, pa, pb, status, s);
   else

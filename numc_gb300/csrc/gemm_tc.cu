@@ -66,6 +66,21 @@ int sm_count() {
   return cached[dev];
 }
 
+int pair_tile_columns(int64_t M, int64_t N) {
+  const int64_t pairs = std::max(1, sm_count() / 2), tm = (M + 255) / 256;
+  int best = 256;
+  int64_t t_best = 0;
+  for (int bn = 256; bn >= 160; bn -= 32) {
+    const int64_t rounds = (tm * ((N + bn - 1) / bn) + pairs - 1) / pairs;
+    const int64_t t = rounds * (bn + 16);   // 16: a tile's own start and end
+    if (bn == 256 || t < t_best) {
+      best = bn;
+      t_best = t;
+    }
+  }
+  return best;
+}
+
 // Programmatic dependent launch of the GEMM kernels after their operand
 // passes (on unless NUMC_CUDA_PDL=0; read once).
 bool pdl_enabled() {
@@ -430,7 +445,8 @@ template <int BN, int STAGES, int PLANES, int FLUSH, bool F16, int CTAS>
 __global__ void __launch_bounds__(SplitCfg<BN, STAGES, PLANES, FLUSH, CTAS>::THREADS, 1)
 split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB,
            float *__restrict__ C, int64_t rso, int64_t cso, int M, int N, int num_kb,
-           int tiles_m, int tiles_n, int vec4, unsigned *status, Fallback fb, WaitCfg wc) {
+           int tiles_m, int tiles_n, int bn, int vec4, unsigned *status, Fallback fb,
+           WaitCfg wc) {
   using Cfg = SplitCfg<BN, STAGES, PLANES, FLUSH, CTAS>;
   using P = Products<PLANES>;
   constexpr bool PAIR = CTAS == 2;
@@ -459,7 +475,7 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
     const int gm = min(tiles_m - first_m, GM);
     const int local = t - group * GM * tiles_n;
     m0 = (first_m + local % gm) * (kBM * CTAS);
-    n0 = (local / gm) * BN;
+    n0 = (local / gm) * bn;
   };
 
   if (threadIdx.x == 0) {
@@ -496,7 +512,7 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
       for (int t = first_tile; t < ntiles && live; t += tile_step) {
         int m0, n0;
         tile_origin(t, m0, n0);
-        const int ma = m0 + (int)rank * kBM, nb = n0 + (int)rank * Cfg::BN_CTA;
+        const int ma = m0 + (int)rank * kBM, nb = n0 + (int)rank * (bn / CTAS);
         for (int kb = 0; kb < num_kb; kb++, g++) {
           const int s = g % STAGES;
           if (g >= STAGES &&
@@ -509,7 +525,8 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
           const uint32_t fbar = tc::smem_u32(&full[s]);
           const uint32_t st = tc::smem_u32(smem + s * Cfg::STAGE_BYTES);
           // The even CTA's full barrier counts the bytes of both CTAs.
-          if (leader) tc::mbar_arrive_expect_tx(fbar, CTAS * Cfg::STAGE_BYTES);
+          if (leader) tc::mbar_arrive_expect_tx(
+                fbar, CTAS * PLANES * (Cfg::A_BYTES + (uint32_t)(bn / CTAS) * kBK * 2));
           const int k = kb * kBK;
           if constexpr (PAIR) {
             const uint32_t fbar_leader = tc::mapa_shared(fbar, 0);
@@ -533,8 +550,9 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
   } else if (warp == 1) {
     if (leader) {
       const bool lead = tc::elect_one();
-      constexpr uint32_t idesc =
-          F16 ? tc::idesc_f16_f32(kBM * CTAS, BN) : tc::idesc_bf16_f32(kBM * CTAS, BN);
+      const uint32_t idesc =
+          (F16 ? tc::idesc_f16_f32(kBM * CTAS, 0) : tc::idesc_bf16_f32(kBM * CTAS, 0)) |
+          (uint32_t)(bn >> 3) << 17;
       int g = 0, chunk = 0;   // stage and chunk counters across tiles
       bool live = true;
       for (int t = first_tile; t < ntiles && live; t += tile_step) {
@@ -637,10 +655,11 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
       }
       if (!ok) break;
 
+      const int Nt = min(N, n0 + bn);   // the tile's columns end here
       // (a pair's odd CTA may lie wholly below the last row: no flag there)
       bool nonfinite = mr < M && fb.flags_a[mr / kBM] == fb.gen;
 #pragma unroll 1
-      for (int c = n0 / 64; c < (n0 + BN) / 64 && c * 64 < N; c++)
+      for (int c = n0 / 64; c * 64 < Nt; c++)
         nonfinite |= fb.flags_b[c] == fb.gen;
       // The warp's staging buffer: first its 64 column scale exponents
       // (float16 planes; one load per lane and half, read back as
@@ -652,8 +671,8 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
         static_assert(Cfg::EPI_STAGE, "float16 planes stage their epilogue");
         if (!nonfinite) {
           const int lc = n0 + cbase + lane;
-          ((int *)stage)[lane] = lc < N ? f16_scale_exp(fb.max_b[lc]) : 0;
-          ((int *)stage)[lane + 32] = lc + 32 < N ? f16_scale_exp(fb.max_b[lc + 32]) : 0;
+          ((int *)stage)[lane] = lc < Nt ? f16_scale_exp(fb.max_b[lc]) : 0;
+          ((int *)stage)[lane + 32] = lc + 32 < Nt ? f16_scale_exp(fb.max_b[lc + 32]) : 0;
           __syncwarp();
         }
       }
@@ -671,13 +690,13 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
 #pragma unroll
             for (int j = 0; j < 32; j++) {
               const int col = n0 + c0 + j;
-              const float bv = col < N ? brow[(int64_t)col * fb.csb] : 0.0f;
+              const float bv = col < Nt ? brow[(int64_t)col * fb.csb] : 0.0f;
               f[j] = __fmaf_rn(av, bv, f[j]);
             }
           }
 #pragma unroll
           for (int j = 0; j < 32; j++)
-            if (n0 + c0 + j < N)
+            if (n0 + c0 + j < Nt)
               C[(int64_t)row * rso + (int64_t)(n0 + c0 + j) * cso] =
                   fb.bias ? __fadd_rn(f[j], fb.bias[(int64_t)(n0 + c0 + j) * fb.bias_stride]) : f[j];
         }
@@ -710,19 +729,19 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
 #pragma unroll
             for (int j = 0; j < CW; j++) {
               const int col = n0 + cbase + j;
-              if (col < N) acc[j] = __fadd_rn(acc[j], fb.bias[(int64_t)col * fb.bias_stride]);
+              if (col < Nt) acc[j] = __fadd_rn(acc[j], fb.bias[(int64_t)col * fb.bias_stride]);
             }
           }
         }
         if (Cfg::EPI_STAGE && cso == 1) {   // warp-uniform: every lane stores
           __syncwarp();
-          store_rows_coalesced<CW>(acc, stage, C, rso, mr + quad * 32, n0 + cbase, M, N, lane);
+          store_rows_coalesced<CW>(acc, stage, C, rso, mr + quad * 32, n0 + cbase, M, Nt, lane);
         } else if (row < M) {
           float *crow = C + (int64_t)row * rso;
 #pragma unroll
           for (int c0 = 0; c0 < CW; c0 += 32) {
             const int nb = n0 + cbase + c0;
-            if (vec4 && nb + 32 <= N) {
+            if (vec4 && nb + 32 <= Nt) {
               float4 *p = reinterpret_cast<float4 *>(crow + nb);
 #pragma unroll
               for (int j = 0; j < 8; j++)
@@ -731,7 +750,7 @@ split_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUten
             } else {
 #pragma unroll
               for (int j = 0; j < 32; j++)
-                if (nb + j < N) crow[(int64_t)(nb + j) * cso] = acc[c0 + j];
+                if (nb + j < Nt) crow[(int64_t)(nb + j) * cso] = acc[c0 + j];
             }
           }
         }
@@ -895,6 +914,26 @@ cudaError_t launch_split_pass(const SplitLayout &L, const SplitBufs &b, const Ge
   return e != cudaSuccess ? e : split_b(L, b, g, gen, s);
 }
 
+// The forced output tile width of the float16-plane GEMM (NUMC_CUDA_SPLIT_TILE
+// = 64, 128 or 256, read once), or 0.
+int forced_tile() {
+  static const int v = [] {
+    const char *e = getenv("NUMC_CUDA_SPLIT_TILE");
+    const int t = e ? atoi(e) : 0;
+    return t == 64 || t == 128 || t == 256 ? t : 0;
+  }();
+  return v;
+}
+
+// Columns of the CTA pairs' wide tiles, 256 or a little less: the width whose
+// rounds of tiles over the pairs multiply the fewest columns (the last round of
+// 256-column tiles may occupy few pairs: 4096^2 is 3.4 rounds of them, 4.0 of 224
+// columns; GEMM 261 -> 240 us).
+int wide_tile_columns(const Gemm &g) {
+  if (forced_tile()) return 256;
+  return pair_tile_columns(g.M, g.N);
+}
+
 template <int BN, int STAGES, int PLANES, int FLUSH, bool F16, int CTAS>
 cudaError_t launch_gemm_status(const SplitLayout &L, const SplitBufs &bufs, const Gemm &g,
                                unsigned long long gen, unsigned *status, cudaStream_t s,
@@ -904,13 +943,14 @@ cudaError_t launch_gemm_status(const SplitLayout &L, const SplitBufs &bufs, cons
   cudaError_t e;
   const auto dtype = F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   if ((e = make_tmap_3d(&ta, bufs.pa, dtype, 2, PLANES, g.M, L.Kp, L.Kp, kBM, kBK))) return e;
-  if ((e = make_tmap_3d(&tb, bufs.pb, dtype, 2, PLANES, g.N, L.Kp, L.Kp, Cfg::BN_CTA, kBK)))
+  const int bn = CTAS == 2 && BN == 256 ? wide_tile_columns(g) : BN;
+  if ((e = make_tmap_3d(&tb, bufs.pb, dtype, 2, PLANES, g.N, L.Kp, L.Kp, bn / CTAS, kBK)))
     return e;
   auto kern = split_gemm<BN, STAGES, PLANES, FLUSH, F16, CTAS>;
   static LaunchCache lc;
   if ((e = smem_attr_once(lc, (const void *)kern, Cfg::SMEM))) return e;
   const int tiles_m = (int)((g.M + kBM * CTAS - 1) / (kBM * CTAS));
-  const int tiles_n = (int)((g.N + BN - 1) / BN);
+  const int tiles_n = (int)((g.N + bn - 1) / bn);
   const int vec4 = g.cso == 1 && (g.rso % 4) == 0 && ((uintptr_t)g.c % 16) == 0;
   Fallback fb;
   fb.A = (const float *)g.a;
@@ -938,7 +978,7 @@ cudaError_t launch_gemm_status(const SplitLayout &L, const SplitBufs &bufs, cons
     cfg.attrs = &pdl_attr;
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, kern, ta, tb, (float *)g.c, (int64_t)g.rso, (int64_t)g.cso,
-                           (int)g.M, (int)g.N, num_kb, tiles_m, tiles_n, vec4, status, fb,
+                           (int)g.M, (int)g.N, num_kb, tiles_m, tiles_n, bn, vec4, status, fb,
                            wait_cfg());
     if (e != cudaSuccess) return e;
   } else {
@@ -962,7 +1002,7 @@ cudaError_t launch_gemm_status(const SplitLayout &L, const SplitBufs &bufs, cons
     cfg.gridDim = dim3((unsigned)(CTAS * pairs));
     cfg.numAttrs = 2;
     e = cudaLaunchKernelEx(&cfg, kern, ta, tb, (float *)g.c, (int64_t)g.rso, (int64_t)g.cso,
-                           (int)g.M, (int)g.N, num_kb, tiles_m, tiles_n, vec4, status, fb,
+                           (int)g.M, (int)g.N, num_kb, tiles_m, tiles_n, bn, vec4, status, fb,
                            wait_cfg());
     if (e != cudaSuccess) return e;
   }
@@ -1002,11 +1042,7 @@ constexpr int kF16DefaultFlush = 4;
 // the same for every width.  NUMC_CUDA_SPLIT_TILE=64, 128 or 256 pins it
 // (read once).
 int split_tile_width(const Gemm &g, int ctas) {
-  static const int forced = [] {
-    const char *e = getenv("NUMC_CUDA_SPLIT_TILE");
-    return e ? atoi(e) : 0;
-  }();
-  if (forced == 64 || forced == 128 || forced == 256) return forced;
+  if (const int forced = forced_tile()) return forced;
   const int64_t rows = 128 * ctas;
   const int64_t wide = (g.M + rows - 1) / rows * ((g.N + 255) / 256);
   if (2 * wide >= sm_count() / ctas) return 256;
