@@ -150,12 +150,31 @@ grouped_scale_split(const Prob *__restrict__ probs, const int2 *__restrict__ job
 }
 
 // ---- persistent grouped split GEMM ----------------------------------------------
+//
+// One CTA per SM, one warp each for TMA and MMA, two groups of 8 warps that
+// take the tiles in turn: a tile's rescale and store are as long as a few
+// slabs' MMAs, and a chunk is one slab (float16 planes), so a single group
+// left the four buffers full and the MMAs waiting.  With tile look-ups by
+// lane and the maxima loaded before the first chunk, 2304 problems of 16 to
+// 1024 (24 and 42 tiles a CTA; mostly 1 to 8 slabs): 128 columns 315 -> 211
+// us, 64 columns 269 -> 187.  The planes' loads alone take 145 and 130 (0.6
+// GB each from HBM), the stores 30; the third stage is worth 5.
+
+// K slabs of a CTA's tile i (0 from `mine` on).
+__device__ __forceinline__ int tile_slabs(const Prob *probs, const Tile *tiles, int i, int mine) {
+  if (i >= mine) return 0;
+  const Tile tl = tiles[blockIdx.x + i * gridDim.x];
+  int kb0, kb1;
+  slice_range(probs[tl.prob], tl.ks, kb0, kb1);
+  return kb1 - kb0;
+}
 
 template <int BN, int STAGES, int FLUSH>
 struct Cfg {
   static constexpr uint32_t A_BYTES = kBM * kBK * 2, B_BYTES = BN * kBK * 2;
   static constexpr uint32_t STAGE_BYTES = kPlanes * (A_BYTES + B_BYTES);
-  static constexpr int ACC_WARPS = 8;
+  // two groups of 8 accumulator warps, taking the tiles in turn
+  static constexpr int GROUP_WARPS = 8, ACC_WARPS = 2 * GROUP_WARPS;
   // ring, barriers, and per accumulator warp a staging buffer for coalesced
   // stores
   static constexpr uint32_t SMEM =
@@ -164,7 +183,7 @@ struct Cfg {
   static constexpr int CW = BN / 2;
   static constexpr int THREADS = 64 + 32 * ACC_WARPS;
   static_assert(SMEM <= 232448, "shared memory");
-  static_assert((2 * STAGES + 2 * NBUF + 1) * 8 + 4 <= 256, "barrier space");
+  static_assert((2 * STAGES + 2 * NBUF + 3) * 8 + 4 <= 256, "barrier space");
 };
 
 template <int BN, int STAGES, int FLUSH, bool F16>
@@ -180,17 +199,19 @@ grouped_split_gemm(const CUtensorMap *__restrict__ tmaps, const Prob *__restrict
   uint64_t *full = bars, *empty = bars + STAGES;
   uint64_t *tfull = bars + 2 * STAGES, *tempty = tfull + NBUF;
   uint64_t *drain = tempty + NBUF;   // all issued MMAs complete
-  uint32_t *tmem_slot = (uint32_t *)(drain + 1);
+  uint64_t *turn = drain + 1;        // per accumulator group: its tile's last chunk is drained
+  uint32_t *tmem_slot = (uint32_t *)(turn + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    for (int b = 0; b < 2; b++) tc::mbar_init(tc::smem_u32(&turn[b]), C_::GROUP_WARPS);
     for (int s = 0; s < STAGES; s++) {
       tc::mbar_init(tc::smem_u32(&full[s]), 1);
       tc::mbar_init(tc::smem_u32(&empty[s]), 1);
     }
     for (int b = 0; b < NBUF; b++) {
       tc::mbar_init(tc::smem_u32(&tfull[b]), 1);
-      tc::mbar_init(tc::smem_u32(&tempty[b]), C_::ACC_WARPS);
+      tc::mbar_init(tc::smem_u32(&tempty[b]), C_::GROUP_WARPS);
     }
     tc::mbar_init(tc::smem_u32(drain), 1);
     tc::fence_barrier_init();
@@ -201,17 +222,26 @@ grouped_split_gemm(const CUtensorMap *__restrict__ tmaps, const Prob *__restrict
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
+  // Tile i of this CTA is tiles[blockIdx.x + i * gridDim.x].  Every warp looks
+  // up 32 of its tiles at once, one a lane (their list entry, problem and K
+  // slabs are a chain of loads of a few hundred ns each).
+  const int mine = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+
   if (warp == 0) {
-    if (lane == 0) {
-      int g = 0;
-      bool live = true;
-      for (int t = blockIdx.x; t < ntiles && live; t += gridDim.x) {
-        const Tile tl = tiles[t];
-        int kb0, kb1;
+    int g = 0;
+    bool live = true;
+    Tile tl;
+    int kb0 = 0, kb1 = 0;
+    for (int i = 0; i < mine && live; i++) {
+      if (i % 32 == 0 && i + lane < mine) {
+        tl = tiles[blockIdx.x + (i + lane) * gridDim.x];
         slice_range(probs[tl.prob], tl.ks, kb0, kb1);
+        tc::tensormap_acquire(tmaps + 2 * tl.prob);
+        tc::tensormap_acquire(tmaps + 2 * tl.prob + 1);
+      }
+      // the lane that acquired the tile's tensor maps loads it
+      if (lane == i % 32) {
         const CUtensorMap *ta = tmaps + 2 * tl.prob, *tb = ta + 1;
-        tc::tensormap_acquire(ta);
-        tc::tensormap_acquire(tb);
         for (int kb = kb0; kb < kb1; kb++, g++) {
           const int s = g % STAGES;
           if (g >= STAGES &&
@@ -232,24 +262,23 @@ grouped_split_gemm(const CUtensorMap *__restrict__ tmaps, const Prob *__restrict
           }
         }
       }
+      g = __shfl_sync(0xffffffffu, g, i % 32);
+      live = __shfl_sync(0xffffffffu, live, i % 32);
     }
-    __syncwarp();
   } else if (warp == 1) {
     {
       const bool lead = tc::elect_one();
       constexpr uint32_t idesc = F16 ? tc::idesc_f16_f32(kBM, BN) : tc::idesc_bf16_f32(kBM, BN);
-      int g = 0, chunk = 0;
+      int g = 0, chunk = 0, slabs32 = 0;
       bool live = true;
-      for (int t = blockIdx.x; t < ntiles && live; t += gridDim.x) {
-        int kb0, kb1;
-        slice_range(probs[tiles[t].prob], tiles[t].ks, kb0, kb1);
-        // loaded values made uniform for the compiler too
-        kb1 = (int)__reduce_max_sync(0xffffffffu, (unsigned)(kb1 - kb0));
-        kb0 = 0;
-        for (int kb = kb0; kb < kb1; kb++, g++) {
+      for (int i = 0; i < mine && live; i++) {
+        if (i % 32 == 0) slabs32 = tile_slabs(probs, tiles, i + lane, mine);
+        // uniform for the compiler too
+        const int nkb = (int)__reduce_max_sync(0xffffffffu, lane == i % 32 ? slabs32 : 0);
+        for (int kb = 0; kb < nkb; kb++, g++) {
           const int s = g % STAGES, buf = chunk % NBUF;
-          const bool cstart = (kb - kb0) % FLUSH == 0;
-          const bool cend = (kb - kb0) % FLUSH == FLUSH - 1 || kb == kb1 - 1;
+          const bool cstart = kb % FLUSH == 0;
+          const bool cend = kb % FLUSH == FLUSH - 1 || kb == nkb - 1;
           if (cstart && chunk >= NBUF &&
               !tc::mbar_wait_warp(tc::smem_u32(&tempty[buf]), ((chunk / NBUF) & 1) ^ 1,
                                      status, kStatusTimeoutMma, wc.limit_ns)) {
@@ -292,41 +321,67 @@ grouped_split_gemm(const CUtensorMap *__restrict__ tmaps, const Prob *__restrict
     __syncwarp();
   } else {
     constexpr int CW = C_::CW;
-    const int quad = warp & 3, half = (warp - 2) >> 2;
+    // Two groups of 8 warps: while one scales and stores a tile, the other
+    // already drains the next one's chunks.
+    const int quad = warp & 3, half = ((warp - 2) >> 2) & 1, group = (warp - 2) >> 3;
     const int cbase = half * CW;
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
-    int chunk = 0;
+    int chunk = 0, slabs32 = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-      const Tile tl = tiles[t];
+    for (int i = 0; i < mine && ok; i++) {
+      if (i % 32 == 0) slabs32 = tile_slabs(probs, tiles, i + lane, mine);
+      const int nchunks = (__shfl_sync(0xffffffffu, slabs32, i % 32) + FLUSH - 1) / FLUSH;
+      if ((i & 1) != group) {
+        chunk += nchunks;
+        continue;
+      }
+      const Tile tl = tiles[blockIdx.x + i * gridDim.x];
       const Prob &P = probs[tl.prob];
       const int row = tl.m0 + quad * 32 + lane;
+      // flags and maxima, loaded while the first chunk is multiplied
+      bool nonfinite = false;
+      unsigned max_row = 0, max_lo = 0, max_hi = 0;
+      if (P.splits <= 1) {
+        nonfinite = P.flags_a[tl.m0 / kBM] == gen;
+        for (int c = tl.n0 / 64; c < (tl.n0 + BN) / 64 && c * 64 < P.N; c++)
+          nonfinite |= P.flags_b[c] == gen;
+        if (F16) {
+          const int lc = tl.n0 + cbase + lane;
+          if (row < P.M) max_row = P.max_a[row];
+          if (lc < P.N) max_lo = P.max_b[lc];
+          if (CW > 32 && lc + 32 < P.N) max_hi = P.max_b[lc + 32];
+        }
+      }
       float acc[CW];
 #pragma unroll
       for (int j = 0; j < CW; j++) acc[j] = 0.0f;
-      int kb0, kb1;
-      slice_range(P, tl.ks, kb0, kb1);
-      const int nchunks = (kb1 - kb0 + FLUSH - 1) / FLUSH;
-      for (int c = 0; c < nchunks; c++, chunk++) {
+      // The other group's tile is drained first: a wait on a chunk's barrier can
+      // tell only consecutive uses of its buffer apart.
+      if (i > 0) ok = tc::mbar_wait_warp(tc::smem_u32(&turn[group ^ 1]), ((i - 1) >> 1) & 1, status,
+                                         kStatusTimeoutEpilogue, wc.limit_ns);
+      for (int c = 0; c < nchunks && ok; c++, chunk++) {
         const int buf = chunk % NBUF;
         ok = tc::mbar_wait_bounded(tc::smem_u32(&tfull[buf]), (chunk / NBUF) & 1, status,
                                    kStatusTimeoutEpilogue, wc.limit_ns);
         ok = __all_sync(0xffffffffu, ok);   // tcgen05.ld below is warp-collective
         if (!ok) break;
         tc::tc_fence_after();
-        uint32_t r[CW];
+        // 16 columns at a time: 96 registers a thread hold no more
 #pragma unroll
-        for (int c0 = 0; c0 < CW; c0 += 32)
-          tc::tmem_ld_32x32b_x32(tmem + lane_off + buf * BN + cbase + c0,
-                                 *reinterpret_cast<uint32_t(*)[32]>(&r[c0]));
-        tc::tmem_ld_wait();
+        for (int c0 = 0; c0 < CW; c0 += 16) {
+          uint32_t r[16];
+          tc::tmem_ld_32x32b_x16(tmem + lane_off + buf * BN + cbase + c0, r);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; j++)
+            acc[c0 + j] = __fadd_rn(acc[c0 + j], __uint_as_float(r[j]));
+        }
         tc::tc_fence_before();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(tc::smem_u32(&tempty[buf]));
-#pragma unroll
-        for (int j = 0; j < CW; j++) acc[j] = __fadd_rn(acc[j], __uint_as_float(r[j]));
       }
       if (!ok) break;
+      if (lane == 0) tc::mbar_arrive(tc::smem_u32(&turn[group]));
       if (P.splits > 1) {
         // split-K: this slice's unscaled partial sums; the ordered
         // reduction adds the slices, rescales and checks the flags
@@ -337,17 +392,12 @@ grouped_split_gemm(const CUtensorMap *__restrict__ tmaps, const Prob *__restrict
         __syncwarp();
         continue;
       }
-      bool nonfinite = P.flags_a[tl.m0 / kBM] == gen;
-      for (int c = tl.n0 / 64; c < (tl.n0 + BN) / 64 && c * 64 < P.N; c++)
-        nonfinite |= P.flags_b[c] == gen;
       if (F16 && !nonfinite) {
         // acc * 2^-(s_row + s_col), correctly rounded (see gemm_tc.cu); the
         // warp's column exponents are loaded once and broadcast (every lane
         // runs this, rows past M included: nonfinite is the warp's tile's)
-        const int lc = tl.n0 + cbase + lane;
-        const int eb_lo = lc < P.N ? f16_scale_exp(P.max_b[lc]) : 0;
-        const int eb_hi = (CW > 32 && lc + 32 < P.N) ? f16_scale_exp(P.max_b[lc + 32]) : 0;
-        const int sa = row < P.M ? f16_scale_exp(P.max_a[row]) : 0;
+        const int eb_lo = f16_scale_exp(max_lo), eb_hi = f16_scale_exp(max_hi);
+        const int sa = f16_scale_exp(max_row);
 #pragma unroll
         for (int j = 0; j < CW; j++) {
           const int e = -(sa + __shfl_sync(0xffffffffu, j < 32 ? eb_lo : eb_hi, j & 31));

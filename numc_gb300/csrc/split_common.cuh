@@ -583,6 +583,7 @@ __device__ __forceinline__ void store_rows_coalesced(const float (&v)[W], float 
   static_assert(W % 16 == 0, "16-column blocks");
 #pragma unroll
   for (int c0 = 0; c0 < W; c0 += 16) {
+    if (row0 >= M || col0 + c0 >= N) break;   // nothing (more) to store
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const int qs = q ^ ((lane >> 1) & 3);
@@ -595,7 +596,7 @@ __device__ __forceinline__ void store_rows_coalesced(const float (&v)[W], float 
     float *dst = C + (int64_t)(row0 + r1) * rso + (col0 + c0 + c);
     int rows_left = M - (row0 + r1);
     const bool col_ok = col0 + c0 + c < N;
-#pragma unroll 1
+#pragma unroll 4
     for (int rr = 0; rr < 32; rr += 2, dst += 2 * rso, rows_left -= 2) {
       const int r = rr + r1;
       const float x = stage[r * 16 + (((c >> 2) ^ ((r >> 1) & 3)) << 2) + (c & 3)];
