@@ -310,16 +310,6 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t lo) {
   return (uint64_t)kSdescHi << 32 | lo;
 }
 
-// Contiguous copy of `bytes` (a multiple of 16) into shared memory.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes,
-                                          uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          dst),
-      "l"((uint64_t)__cvta_generic_to_global(src)), "r"(bytes), "r"(bar)
-      : "memory");
-}
-
 // The S digit planes of n K steps of a block with `rows` of ROWS rows: one copy
 // where the block is full, else a copy per plane (the image holds only its rows),
 // each issued by a lane of its own: one lane took 75 cycles a copy, more than the
@@ -328,9 +318,9 @@ template <int S, int ROWS>
 __device__ __forceinline__ void load_planes(uint32_t dst, const uint16_t *src, int rows, int n,
                                             uint32_t bar, int lane) {
   if (rows == ROWS) {
-    if (lane == 0) bulk_load(dst, src, n * S * ROWS * kRowBytes, bar);
+    if (lane == 0) tc::bulk_load(dst, src, n * S * ROWS * kRowBytes, bar);
   } else if (lane < n * S) {
-    bulk_load(dst + lane * ROWS * kRowBytes, src + (int64_t)lane * rows * kKS, rows * kRowBytes,
+    tc::bulk_load(dst + lane * ROWS * kRowBytes, src + (int64_t)lane * rows * kKS, rows * kRowBytes,
               bar);
   }
 }

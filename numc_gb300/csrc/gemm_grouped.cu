@@ -128,25 +128,25 @@ grouped_split(const Prob *__restrict__ probs, const int2 *__restrict__ jobs,
 
 // ---- fused scale and split (float16 planes) --------------------------------------
 
-// One block: kFusedRows rows of one operand (A's rows, or B's columns as the
+// One block: fused_rows(K) rows of one operand (A's rows, or B's columns as the
 // rows of B^T) over the whole of K: each row's largest magnitude (the scale
 // pass's result, stored for the GEMM's final rescale), then the two float16
-// planes, from one launch and one DRAM read of the operand.  jobs[b] =
-// (problem, block), A's blocks first.  kFusedRows and the block body:
-// split_common.cuh.
+// planes, from one launch and one DRAM read of the operand.  jobs[b] holds all
+// that the block needs (one look-up instead of job, then problem: 484 -> 463
+// us).  The block bodies: split_common.cuh.
+inline __host__ __device__ int fused_rows(int K) {
+  return staged_rows(K) ? staged_rows(K) : kFusedRows;
+}
 
 __global__ void __launch_bounds__(256)
-grouped_scale_split(const Prob *__restrict__ probs, const int2 *__restrict__ jobs,
-                    unsigned long long gen) {
-  const int2 job = jobs[blockIdx.x];
-  const Prob &P = probs[job.x];
-  const int a_blocks = (P.M + kFusedRows - 1) / kFusedRows;
-  const bool is_a = job.y < a_blocks;
-  fused_scale_split_rows<false>(is_a ? P.A : P.B, is_a ? P.rsa : P.csb, is_a ? P.csa : P.rsb,
-                         is_a ? P.M : P.N, P.K, P.Kp,
-                         (is_a ? job.y : job.y - a_blocks) * kFusedRows,
-                         is_a ? P.pa : P.pb, is_a ? P.flags_a : P.flags_b, is_a ? kBM : 64,
-                         is_a ? P.max_a : P.max_b, gen);
+grouped_scale_split(const SplitJob *__restrict__ jobs, unsigned *status, unsigned long long gen,
+                    WaitCfg wc) {
+  const SplitJob J = jobs[blockIdx.x];
+  if (staged_rows(J.K))
+    staged_scale_split(J, staged_rows(J.K), status, gen, wc.limit_ns);
+  else
+    fused_scale_split_rows(J.src, J.rs_row, J.rs_k, J.R, J.K, J.Kp, J.r0, J.planes,
+                                  J.flags, J.flag_rows, J.maxbits, gen);
 }
 
 // ---- persistent grouped split GEMM ----------------------------------------------
@@ -546,7 +546,7 @@ struct NumcCudaGemmPlan {
   long long split_jobs;
   bool f16;                       // scaled float16 planes (else bfloat16)
   int2 *d_max_jobs;               // (problem, job) of each scale block (float16 planes)
-  int2 *d_fused_jobs;             // (problem, block) of the fused scale + split pass
+  SplitJob *d_fused_jobs;         // the blocks of the fused scale + split pass
   long long fused_jobs;
   long long max_jobs;
   int n_split_probs;
@@ -696,8 +696,8 @@ int plan_enqueue(NumcCudaGemmPlan *p, cudaStream_t s, unsigned *kernels) {
     ++*kernels;
   }
   if (p->fused_jobs > 0) {
-    grouped_scale_split<<<(unsigned)p->fused_jobs, 256, 0, s>>>(
-        p->d_split_probs, p->d_fused_jobs, p->gen);
+    grouped_scale_split<<<(unsigned)p->fused_jobs, 256, 0, s>>>(p->d_fused_jobs, status, p->gen,
+                                                                  wait_cfg());
     if ((e = cudaGetLastError())) return fail(e, "grouped scale and split");
     ++*kernels;
   }
@@ -878,12 +878,13 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   tiles[kVarSimt].insert(tiles[kVarSimt].end(), simt_small.begin(), simt_small.end());
   // Job tables: (problem, job within it) for every block of the scale,
   // split and remainder passes, so a block finds its problem in one load.
-  std::vector<int2> split_jobs, max_jobs, edge_jobs, fused_jobs;
+  std::vector<int2> split_jobs, max_jobs, edge_jobs;
+  long long n_fused = 0;
   for (size_t q = 0; q < split_idx.size(); q++) {
     const Prob &P = p->probs[split_idx[q]];
     if (p->f16) {   // float16 planes: one fused scale + split pass
-      const long long n = (P.M + kFusedRows - 1) / kFusedRows + (P.N + kFusedRows - 1) / kFusedRows;
-      for (long long j = 0; j < n; j++) fused_jobs.push_back(make_int2((int)q, (int)j));
+      const long long rows = fused_rows(P.K);
+      n_fused += (P.M + rows - 1) / rows + (P.N + rows - 1) / rows;
       continue;
     }
     const long long kt = (P.Kp + kSplitK - 1) / kSplitK;
@@ -921,7 +922,7 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   p->n_split_probs = (int)split_idx.size();
   p->max_jobs = (long long)max_jobs.size();
   p->edge_jobs = (long long)edge_jobs.size();
-  p->fused_jobs = (long long)fused_jobs.size();
+  p->fused_jobs = n_fused;
   p->sk_jobs = (long long)sk_jobs.size();
   p->n_sk_probs = (int)sk_idx.size();
   if (p->split_jobs > 0x7FFFFFFFll || p->max_jobs > 0x7FFFFFFFll || p->edge_jobs > 0x7FFFFFFFll ||
@@ -938,7 +939,7 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   const size_t o_sprobs = off; off = align_up(off + split_idx.size() * sizeof(Prob), 256);
   const size_t o_split_jobs = off; off = align_up(off + split_jobs.size() * sizeof(int2), 256);
   const size_t o_max_jobs = off; off = align_up(off + max_jobs.size() * sizeof(int2), 256);
-  const size_t o_fused_jobs = off; off = align_up(off + fused_jobs.size() * sizeof(int2), 256);
+  const size_t o_fused_jobs = off; off = align_up(off + (size_t)n_fused * sizeof(SplitJob), 256);
   const size_t o_sk = off; off = align_up(off + sk_idx.size() * sizeof(int), 256);
   const size_t o_sk_jobs = off; off = align_up(off + sk_jobs.size() * sizeof(int2), 256);
   const size_t o_edges = off; off = align_up(off + edge_idx.size() * sizeof(int), 256);
@@ -963,7 +964,7 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   p->d_split_probs = (Prob *)(p->dev + o_sprobs);
   p->d_split_jobs = (int2 *)(p->dev + o_split_jobs);
   p->d_max_jobs = (int2 *)(p->dev + o_max_jobs);
-  p->d_fused_jobs = (int2 *)(p->dev + o_fused_jobs);
+  p->d_fused_jobs = (SplitJob *)(p->dev + o_fused_jobs);
   p->d_sk_probs = (int *)(p->dev + o_sk);
   p->d_sk_jobs = (int2 *)(p->dev + o_sk_jobs);
   p->d_edge_probs = (int *)(p->dev + o_edges);
@@ -1011,6 +1012,16 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   }
   std::vector<Prob> sp(split_idx.size());
   for (size_t q = 0; q < split_idx.size(); q++) sp[q] = p->probs[split_idx[q]];
+  std::vector<SplitJob> sj;
+  sj.reserve((size_t)n_fused);
+  if (p->f16)
+    for (const Prob &P : sp) {
+      const int rows = fused_rows(P.K);
+      for (int r0 = 0; r0 < P.M; r0 += rows)
+        sj.push_back(SplitJob{P.A, P.rsa, P.csa, P.pa, P.flags_a, P.max_a, P.M, P.K, P.Kp, r0, kBM});
+      for (int r0 = 0; r0 < P.N; r0 += rows)
+        sj.push_back(SplitJob{P.B, P.csb, P.rsb, P.pb, P.flags_b, P.max_b, P.N, P.K, P.Kp, r0, 64});
+    }
   if ((e = cudaMemcpy(p->d_tmaps, tm.data(), tm.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice)) ||
       (e = cudaMemcpy(p->d_probs, p->probs.data(), count * sizeof(Prob), cudaMemcpyHostToDevice)) ||
       (e = cudaMemcpy(p->d_split_probs, sp.data(), sp.size() * sizeof(Prob), cudaMemcpyHostToDevice)) ||
@@ -1020,8 +1031,8 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
       (!max_jobs.empty() &&
        (e = cudaMemcpy(p->d_max_jobs, max_jobs.data(), max_jobs.size() * sizeof(int2),
                        cudaMemcpyHostToDevice))) ||
-      (!fused_jobs.empty() &&
-       (e = cudaMemcpy(p->d_fused_jobs, fused_jobs.data(), fused_jobs.size() * sizeof(int2),
+      (!sj.empty() &&
+       (e = cudaMemcpy(p->d_fused_jobs, sj.data(), sj.size() * sizeof(SplitJob),
                        cudaMemcpyHostToDevice))) ||
       (!sk_idx.empty() &&
        ((e = cudaMemcpy(p->d_sk_probs, sk_idx.data(), sk_idx.size() * sizeof(int),

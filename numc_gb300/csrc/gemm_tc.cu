@@ -126,7 +126,7 @@ int clusters_once(LaunchCache &lc, const void *kern, const cudaLaunchConfig_t &c
 namespace {
 
 constexpr int kBM = 128, kBK = 64;
-constexpr int kFusedMaxKp = 1024;   // single problems: fused scale + split up to this K
+constexpr int kFusedMaxKp = 1536;   // single problems: fused scale + split up to this K
 
 __host__ __device__ inline int64_t round_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
@@ -343,22 +343,18 @@ bool launch_split_cols(const float *src, int64_t rs_k, int64_t R, int64_t K, int
   return go(scale_split_cols<2>, lc2);
 }
 
-// Both operands of one float16-plane split through fused_scale_split_rows:
-// blocks [0, a_blocks) take 16 rows of A each, the
-// rest 16 columns of B.  One launch replaces two zeroings of the maxima,
-// two absmax passes and two split passes.
+// Both operands of one float16-plane split, `rows` rows a block: blocks [0,
+// a_blocks) take rows of A, the rest columns of B.  One launch replaces two
+// zeroings of the maxima, two absmax passes and two split passes.
 __global__ void __launch_bounds__(256)
-scale_split_pair(const float *A, int64_t rsa, int64_t csa, int M, const float *B,
-                 int64_t rsb, int64_t csb, int N, int K, int Kp, uint16_t *pa, uint16_t *pb,
-                 unsigned long long *fa, unsigned long long *fbl, unsigned *max_a,
-                 unsigned *max_b, unsigned long long gen) {
+scale_split_pair(const SplitJob a, const SplitJob b, int rows, unsigned *status,
+                 unsigned long long gen, WaitCfg wc) {
   tc::griddep_launch_dependents();   // the GEMM may launch and set up meanwhile
-  const int a_blocks = (M + kFusedRows - 1) / kFusedRows;
+  const int a_blocks = (a.R + rows - 1) / rows;
   const bool is_a = (int)blockIdx.x < a_blocks;
-  fused_scale_split_rows<true>(is_a ? A : B, is_a ? rsa : csb, is_a ? csa : rsb, is_a ? M : N, K, Kp,
-                         (is_a ? (int)blockIdx.x : (int)blockIdx.x - a_blocks) * kFusedRows,
-                         is_a ? pa : pb, is_a ? fa : fbl, is_a ? kBM : 64, is_a ? max_a : max_b,
-                         gen);
+  SplitJob J = is_a ? a : b;
+  J.r0 = (is_a ? (int)blockIdx.x : (int)blockIdx.x - a_blocks) * rows;
+  staged_scale_split(J, rows, status, gen, wc.limit_ns);
 }
 
 // ---- pass 2: the tcgen05 GEMM ------------------------------------------------
@@ -896,17 +892,19 @@ cudaError_t split_b(const SplitLayout &L, const SplitBufs &b, const Gemm &g,
 }
 
 // Launch the split pass of both operands: for float16 planes with K up to
-// kFusedMaxKp one fused scale + split launch over both, else a scale pass
-// and a split pass per operand (large operands: the fused pass's second read
-// would miss L2 like the split pass's does, and the two-pass kernels move
-// 16-byte vectors).
+// kFusedMaxKp (what staged_rows() takes) one fused scale + split launch over
+// both, else a scale pass and a split pass per operand.
 cudaError_t launch_split_pass(const SplitLayout &L, const SplitBufs &b, const Gemm &g,
                               unsigned long long gen, cudaStream_t s) {
   if (L.f16 && L.Kp <= kFusedMaxKp && g.M < (1ll << 30) && g.N < (1ll << 30)) {
-    const int64_t blocks = (g.M + kFusedRows - 1) / kFusedRows + (g.N + kFusedRows - 1) / kFusedRows;
+    const int K = (int)g.K, rows = staged_rows_for(K, g.M + g.N);
+    const int64_t blocks = (g.M + rows - 1) / rows + (g.N + rows - 1) / rows;
     scale_split_pair<<<(unsigned)blocks, 256, 0, s>>>(
-        (const float *)g.a, g.rsa, g.csa, (int)g.M, (const float *)g.b, g.rsb, g.csb, (int)g.N,
-        (int)g.K, (int)L.Kp, b.pa, b.pb, b.flags_a, b.flags_b, b.max_a, b.max_b, gen);
+        SplitJob{(const float *)g.a, g.rsa, g.csa, b.pa, b.flags_a, b.max_a, (int)g.M, K,
+                 (int)L.Kp, 0, kBM},
+        SplitJob{(const float *)g.b, g.csb, g.rsb, b.pb, b.flags_b, b.max_b, (int)g.N, K,
+                 (int)L.Kp, 0, 64},
+        rows, status_word(), gen, wait_cfg());
     count_launch();
     return cudaGetLastError();
   }

@@ -16,6 +16,9 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "status.h"
+#include "tc_common.cuh"
+
 namespace numc_k {
 
 // Scale exponent of a row whose largest magnitude has float32 bits
@@ -343,8 +346,8 @@ __device__ __forceinline__ void split_tile(const float *__restrict__ src, int64_
 // columns as B^T's rows).  Pass 1 reads the rows for their maxima; pass 2
 // reads them again (from L2: a block's rows are at most kFusedRows x K
 // elements) and writes the two float16 planes — one launch and one DRAM read
-// of the operand instead of the absmax and split passes.  No shared-memory
-// staging, so many blocks fit on an SM and K is unbounded.  Writes
+// of the operand instead of the absmax and split passes.  For grouped problems
+// whose K is beyond staged_rows(); no staging, so K is unbounded.  Writes
 // maxbits[row] directly (no zeroing first) and, for a non-finite value,
 // flags[r0 / flag_rows] = gen.  Same arithmetic as split_tile<2, true>.
 // Pass 1 layout: k contiguous (rs_k == 1): 16 threads per row along k;
@@ -354,7 +357,6 @@ __device__ __forceinline__ void split_tile(const float *__restrict__ src, int64_
 // written in 128-byte runs (B's second read comes from L2 in 4-byte pieces).
 constexpr int kFusedRows = 16;
 
-template <bool STASH>
 __device__ __forceinline__ void fused_scale_split_rows(
     const float *__restrict__ src, int64_t rs_row, int64_t rs_k, int R, int K, int Kp, int r0,
     uint16_t *__restrict__ planes, unsigned long long *flags, int flag_rows,
@@ -411,13 +413,7 @@ __device__ __forceinline__ void fused_scale_split_rows(
   }
   if (__syncthreads_or(bad) && tid == 0) flags[r0 / flag_rows] = gen;
 
-  // Pass 2: thread (r2, q) converts k = 4 q + 64 i .. +3 of row r2.  Rows
-  // contiguous along k are read in place; otherwise (the columns of a
-  // row-major B) with STASH each 64-deep chunk of the 16 rows is first read
-  // with the lanes along the rows (64 contiguous bytes per k) into shared
-  // memory (measured faster for one large problem: 512^3 split 18.2 ->
-  // 17.8 us), without it read in place (faster for the grouped launch of
-  // many small problems, whose blocks then sync less: 1.77 -> 1.70 ms).
+  // Pass 2: thread (r2, q) converts k = 4 q + 64 i .. +3 of row r2, read in place.
   const int r2 = tid / 16, q = tid % 16;
   const bool live2 = r0 + r2 < R;
   const int sexp = f16_scale_exp(rowmax[r2]);
@@ -443,22 +439,7 @@ __device__ __forceinline__ void fused_scale_split_rows(
       *reinterpret_cast<uint2 *>(dst + pl * plane_elems + k) = w;
     }
   };
-  if (STASH && !along_k) {
-    __shared__ float stash[kFusedRows][64 + 1];
-    for (int k0 = 0; k0 < Kp; k0 += 64) {
-      __syncthreads();   // the previous chunk's reads of the stash are done
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int kk = (tid >> 4) + 16 * t, k = k0 + kk;
-        stash[r][kk] = live && k < K ? p[(int64_t)k * rs_k] : 0.0f;
-      }
-      __syncthreads();
-      float rem[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) rem[t] = stash[r2][4 * q + t];
-      if (live2) convert_store(rem, k0 + 4 * q);
-    }
-  } else if (live2) {
+  if (live2) {
     const float *p2 = src + (int64_t)(r0 + r2) * rs_row;
 #pragma unroll 2
     for (int k = 4 * q; k < Kp; k += 64) {
@@ -472,6 +453,178 @@ __device__ __forceinline__ void fused_scale_split_rows(
       }
       convert_store(rem, k);
     }
+  }
+}
+
+// ---- fused scale and split, rows staged in shared memory ------------------------
+//
+// The same work with each element read from global memory once: a block's rows
+// (about 32 KB) come into shared memory, then a warp takes the maximum of one
+// row, converts it and writes both planes 128 bytes at a time.  Rows without
+// gaps between them arrive as one bulk copy; others contiguous along k by
+// cp.async of the warp that converts them, so that no barrier is needed; the
+// columns of a row-major B with the lanes along up to 16 of them, at a pitch
+// that spreads 32 lanes' stores over the banks.  cp.async of 4 bytes goes
+// through L1, whose share of the memory bounds the bytes in flight: six blocks
+// on an SM were slower than five (499 against 447 us below), and so were two
+// stages a block (565).  Measured, us before (two reads, no staging) and after:
+// 2304 grouped problems of 16 to 1024 (1.2 GB) 600 / 447 (5.4 TB/s read and
+// written); whole split GEMMs 512^3 14.7 / 13.1, 1024^3 23.3 / 19.5, 256 x
+// 1000 x 256 22.8 / 17.4, 1536 x 700 x 2100 22.9 / 21.4, 3000 x 1000 x 2500
+// 53.7 / 48.0.  With 4 rows a block (K above 1024) a B column set is 16 bytes
+// wide: 2048 x 1100 x 2048 42.8 / 37.3, 512 x 1500 x 512 23.2 / 23.1, but
+// 2048^3 58.2 / 61.8, so K stops at 1536.
+__host__ __device__ inline int staged_rows(int K) {
+  return K <= 256 ? 32 : K <= 512 ? 16 : K <= 1024 ? 8 : K <= 1536 ? 4 : 0;   // 0: K too long
+}
+// Rows a block for `total` rows in all: fewer, down to 8, while that leaves the
+// device under four blocks an SM (512^3 with 16 rows 13.5 us, with 8 13.1).
+inline int staged_rows_for(int K, int64_t total) {
+  int rows = staged_rows(K);
+  while (rows > 8 && total / rows < 608) rows /= 2;
+  return rows;
+}
+constexpr int kStagedFloats = 32 * 258 + 4;
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(float *dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+
+// A block's rows of one operand.
+struct alignas(16) SplitJob {
+  const float *src;
+  int64_t rs_row, rs_k;
+  uint16_t *planes;
+  unsigned long long *flags;
+  unsigned *maxbits;
+  int R, K, Kp, r0, flag_rows;
+};
+__device__ __forceinline__ int staged_pitch(int rows) {
+  return rows == 32 ? 258 : rows == 16 ? 514 : rows == 8 ? 1028 : 2056;
+}
+
+// Starts the copies of the block's rows to `stage` (kStagedFloats floats).
+__device__ __forceinline__ void staged_load(const SplitJob &J, int rows, float *stage) {
+  const int pitch = staged_pitch(rows), K = J.K;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (J.rs_k == 1) {
+    const bool pairs = (J.rs_row & 1) == 0 && (reinterpret_cast<uintptr_t>(J.src) & 7) == 0;
+    for (int r = warp; r < rows && J.r0 + r < J.R; r += 8) {
+      const float *row = J.src + (int64_t)(J.r0 + r) * J.rs_row;
+      float *dst = stage + r * pitch;
+      int k0 = 0;
+      if (pairs) {
+        k0 = K & ~1;
+#pragma unroll 4
+        for (int k = 2 * lane; k < k0; k += 64) copy_async<8>(dst + k, row + k);
+      }
+#pragma unroll 4
+      for (int k = k0 + lane; k < K; k += 32) copy_async<4>(dst + k, row + k);
+    }
+  } else {
+    const int across = min(rows, 16), r1 = tid % across, ks = 256 / across;
+    const int64_t rs_k = J.rs_k;
+    for (int r = r1; r < rows && J.r0 + r < J.R; r += across) {
+      const float *col = J.src + (int64_t)(J.r0 + r) * J.rs_row;
+      float *dst = stage + r * pitch;
+#pragma unroll 8
+      for (int k = tid / across; k < K; k += ks) copy_async<4>(dst + k, col + (int64_t)k * rs_k);
+    }
+  }
+}
+
+// The same for rows without gaps (rs_k == 1, rs_row == K): one bulk copy of
+// whole 16 bytes, the elements before and after it by plain loads.  `bar`: an
+// mbarrier initialised for one arrival; every thread waits for it and then for
+// the block.  Returns the first row's offset in the stage.
+__device__ __forceinline__ int staged_load_bulk(const SplitJob &J, int rows, float *stage,
+                                                uint32_t bar) {
+  const float *src = J.src + (int64_t)J.r0 * J.K;
+  const int n = min(rows, J.R - J.r0) * J.K;
+  const int mis = (int)(reinterpret_cast<uintptr_t>(src) >> 2) & 3;   // dst as aligned as src
+  const int head = min(n, (4 - mis) & 3), body = (n - head) & ~3;
+  const int t = threadIdx.x;
+  if (t == 0) {
+    tc::mbar_arrive_expect_tx(bar, body * 4);
+    if (body)
+      tc::bulk_load((uint32_t)__cvta_generic_to_shared(stage + mis + head), src + head, body * 4, bar);
+  } else if (t >= 32 && t - 32 < head) {
+    stage[mis + t - 32] = src[t - 32];
+  } else if (t >= 64 && head + body + t - 64 < n) {
+    stage[mis + head + body + t - 64] = src[head + body + t - 64];
+  }
+  return mis;
+}
+
+// Maxima and planes of the rows in `stage`, the first at `off`, `pitch` apart.
+__device__ __forceinline__ void staged_convert(const SplitJob &J, int rows, const float *stage,
+                                               int off, int pitch, unsigned long long gen) {
+  const int K = J.K, Kp = J.Kp;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t plane_elems = (int64_t)J.R * Kp;
+  for (int r = warp; r < rows && J.r0 + r < J.R; r += 8) {
+    const float *row = stage + off + r * pitch;
+    const bool even = ((off + r * pitch) & 1) == 0;
+    unsigned m = 0;
+#pragma unroll 4
+    for (int k = lane; k < K; k += 32) m = max(m, absbits(row[k]));
+    m = __reduce_max_sync(0xffffffffu, m);
+    const bool bad = m >= 0x7f800000u;
+    if (lane == 0) {
+      J.maxbits[J.r0 + r] = m;
+      if (bad) J.flags[J.r0 / J.flag_rows] = gen;
+    }
+    const int s = f16_scale_exp(m), s1 = min(s, 126);
+    const float f1 = exp2_int(s1), f2 = exp2_int(s - s1);   // scale_pow2
+    uint32_t *dst = reinterpret_cast<uint32_t *>(J.planes + (int64_t)(J.r0 + r) * Kp);
+#pragma unroll 2
+    for (int k = 2 * lane; k < Kp; k += 64) {
+      float2 x = make_float2(0.f, 0.f);
+      if (even && k < K) {
+        x = *reinterpret_cast<const float2 *>(row + k);
+      } else if (k < K) {
+        x.x = row[k];
+        x.y = row[k + 1];
+      }
+      if (k + 1 >= K) x.y = 0.f;
+      if (bad) {
+        x.x = isfinite(x.x) ? x.x : 0.f;
+        x.y = isfinite(x.y) ? x.y : 0.f;
+      }
+      x.x = x.x * f1 * f2;
+      x.y = x.y * f1 * f2;
+      const __half2 hi = __float22half2_rn(x);
+      const float2 h = __half22float2(hi);
+      const __half2 lo = __float22half2_rn(make_float2(x.x - h.x, x.y - h.y));
+      dst[k / 2] = *reinterpret_cast<const uint32_t *>(&hi);
+      dst[(plane_elems + k) / 2] = *reinterpret_cast<const uint32_t *>(&lo);
+    }
+  }
+}
+
+// A block's whole job; 256 threads.
+__device__ __forceinline__ void staged_scale_split(const SplitJob &J, int rows, unsigned *status,
+                                                   unsigned long long gen, uint64_t limit_ns) {
+  __shared__ __align__(16) float stage[kStagedFloats];
+  __shared__ uint64_t bar;
+  if (J.rs_k == 1 && J.rs_row == J.K) {
+    if (threadIdx.x == 0) {
+      tc::mbar_init(tc::smem_u32(&bar), 1);
+      tc::fence_barrier_init();
+    }
+    __syncthreads();
+    const int off = staged_load_bulk(J, rows, stage, tc::smem_u32(&bar));
+    const bool ok =
+        tc::mbar_wait_bounded(tc::smem_u32(&bar), 0, status, kStatusTimeoutProducer, limit_ns);
+    if (__syncthreads_and(ok)) staged_convert(J, rows, stage, off, J.K, gen);
+  } else {
+    staged_load(J, rows, stage);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (J.rs_k == 1) __syncwarp();   // a warp converts the rows that it copied
+    else __syncthreads();
+    staged_convert(J, rows, stage, 0, staged_pitch(rows), gen);
   }
 }
 

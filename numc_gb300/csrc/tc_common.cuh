@@ -125,6 +125,17 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap *m) {
                : "memory");
 }
 
+// Contiguous copy of `bytes` (a multiple of 16) into shared memory, counted by
+// the mbarrier `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes,
+                                          uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          dst),
+      "l"((uint64_t)__cvta_generic_to_global(src)), "r"(bytes), "r"(bar)
+      : "memory");
+}
+
 // ---- TMEM ---------------------------------------------------------------------
 
 // Executed by one full warp.  Writes the TMEM base address to *dst_smem.
