@@ -12,8 +12,8 @@
 // the reads, the moves that double A's values into pairs and the copies.
 // Operands arrive by 4-byte cp.async in a three-stage ring (any strides and
 // alignment; 16-byte copies need both).  Measured, us before and after:
-//   1000^3 84 / 61, 2000 x 1999 x 1501 591 / 247, 300 x 2500 x 1700 168 / 108,
-//   2048^3 511 / 370, 8192^3 23834 / 20247 (54 TFLOP/s).
+//   1000^3 84 / 61, 2000 x 1999 x 1501 591 / 244, 300 x 2500 x 1700 168 / 109,
+//   2048^3 511 / 363, 8192^3 23834 / 20247 (54 TFLOP/s).
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
