@@ -346,7 +346,7 @@ bool launch_split_cols(const float *src, int64_t rs_k, int64_t R, int64_t K, int
 // Both operands of one float16-plane split, `rows` rows a block: blocks [0,
 // a_blocks) take rows of A, the rest columns of B.  One launch replaces two
 // zeroings of the maxima, two absmax passes and two split passes.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 5)   // 5: see grouped_scale_split
 scale_split_pair(const SplitJob a, const SplitJob b, int rows, unsigned *status,
                  unsigned long long gen, WaitCfg wc) {
   tc::griddep_launch_dependents();   // the GEMM may launch and set up meanwhile

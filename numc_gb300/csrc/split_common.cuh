@@ -466,13 +466,13 @@ __device__ __forceinline__ void fused_scale_split_rows(
 // columns of a row-major B with the lanes along up to 16 of them, at a pitch
 // that spreads 32 lanes' stores over the banks.  cp.async of 4 bytes goes
 // through L1, whose share of the memory bounds the bytes in flight: six blocks
-// on an SM were slower than five (499 against 447 us below), and so were two
+// on an SM were slower than five (495 against 444 us below), and so were two
 // stages a block (565).  Measured, us before (two reads, no staging) and after:
-// 2304 grouped problems of 16 to 1024 (1.2 GB) 600 / 447 (5.4 TB/s read and
-// written); whole split GEMMs 512^3 14.7 / 13.1, 1024^3 23.3 / 19.5, 256 x
-// 1000 x 256 22.8 / 17.4, 1536 x 700 x 2100 22.9 / 21.4, 3000 x 1000 x 2500
-// 53.7 / 48.0.  With 4 rows a block (K above 1024) a B column set is 16 bytes
-// wide: 2048 x 1100 x 2048 42.8 / 37.3, 512 x 1500 x 512 23.2 / 23.1, but
+// 2304 grouped problems of 16 to 1024 (1.2 GB) 600 / 444 (5.4 TB/s read and
+// written); whole split GEMMs 512^3 14.7 / 13.1, 1024^3 23.3 / 19.0, 256 x
+// 1000 x 256 22.8 / 17.1, 1536 x 700 x 2100 22.9 / 21.2, 3000 x 1000 x 2500
+// 53.7 / 46.6.  With 4 rows a block (K above 1024) a B column set is 16 bytes
+// wide: 2048 x 1100 x 2048 42.8 / 35.8, 512 x 1500 x 512 23.2 / 22.4, but
 // 2048^3 58.2 / 61.8, so K stops at 1536.
 __host__ __device__ inline int staged_rows(int K) {
   return K <= 256 ? 32 : K <= 512 ? 16 : K <= 1024 ? 8 : K <= 1536 ? 4 : 0;   // 0: K too long
@@ -524,13 +524,14 @@ __device__ __forceinline__ void staged_load(const SplitJob &J, int rows, float *
       for (int k = k0 + lane; k < K; k += 32) copy_async<4>(dst + k, row + k);
     }
   } else {
-    const int across = min(rows, 16), r1 = tid % across, ks = 256 / across;
+    const int lg = rows == 4 ? 2 : rows == 8 ? 3 : 4;   // log2 of the rows across
+    const int across = 1 << lg, r1 = tid & (across - 1), ks = 256 >> lg;
     const int64_t rs_k = J.rs_k;
     for (int r = r1; r < rows && J.r0 + r < J.R; r += across) {
       const float *col = J.src + (int64_t)(J.r0 + r) * J.rs_row;
       float *dst = stage + r * pitch;
 #pragma unroll 8
-      for (int k = tid / across; k < K; k += ks) copy_async<4>(dst + k, col + (int64_t)k * rs_k);
+      for (int k = tid >> lg; k < K; k += ks) copy_async<4>(dst + k, col + (int64_t)k * rs_k);
     }
   }
 }
