@@ -1,8 +1,9 @@
 #pragma once
 
-// One output tile of a float32 GEMM on the CUDA cores (gemm_f32.cu): a block
-// computes it in numc's arithmetic from operands copied asynchronously into
-// shared memory; element offsets are 32-bit (fits).
+// One output tile of a float32 GEMM on the CUDA cores, for one problem
+// (gemm_f32.cu) and for many (gemm_grouped.cu): a block computes it in numc's
+// arithmetic from operands copied asynchronously into shared memory; element
+// offsets are 32-bit (fits).
 
 #include "kernels.h"
 #include "simt_common.cuh"
@@ -198,6 +199,23 @@ struct F32Acc {
         const u64 aa = twice(i % 4 == 0 ? v.x : i % 4 == 1 ? v.y : i % 4 == 2 ? v.z : v.w);
 #pragma unroll
         for (int j = 0; j < TN / 2; j++) fma2(acc[i][j], aa, b[k & 1][j]);
+      }
+    }
+  }
+
+  // The first n k steps of a slab, n below its depth.
+  __device__ __forceinline__ void part_slab(const float *As, int n) {
+    const float *a0 = As + row_of(0), *b0 = As + BK * Cfg::APITCH;
+#pragma unroll 1
+    for (int k = 0; k < n; k++, a0 += Cfg::APITCH, b0 += Cfg::BPITCH) {
+      u64 b[TN / 2];
+#pragma unroll
+      for (int j = 0; j < TN; j += 2) b[j / 2] = *reinterpret_cast<const u64 *>(b0 + col_of(j));
+#pragma unroll
+      for (int i = 0; i < TM; i++) {
+        const u64 aa = twice(a0[row_of(i) - row_of(0)]);
+#pragma unroll
+        for (int j = 0; j < TN / 2; j++) fma2(acc[i][j], aa, b[j]);
       }
     }
   }

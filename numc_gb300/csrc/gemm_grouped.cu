@@ -17,9 +17,9 @@
 //      columns): each CTA walks a static share of the variant's tile list;
 //      the TMA ring, the MMA chunk stream and the TMEM buffers run on
 //      across tiles, so a tile's stores overlap the next tile's MMAs,
-//   5. one grouped CUDA-core kernel (FP32 FMA chains, numc's arithmetic)
-//      for problems too small for the tensor path, and for the plain
-//      algorithm.
+//   5. grouped CUDA-core kernels (FP32 FMA chains, numc's arithmetic) for
+//      problems too small for the tensor path, and for the plain algorithm:
+//      one per tile list (128 x 64; 16 x 16 and 32 x 32; numc's unpacked path).
 // The tile lists are ordered by K, largest first, so the static
 // round-robin finishes with short tiles.
 #include <cuda.h>
@@ -38,6 +38,7 @@
 #include <string>
 #include <vector>
 
+#include "f32_tiles.cuh"
 #include "kernels.h"
 #include "numc/cuda.h"
 #include "numc/error.h"
@@ -162,6 +163,14 @@ grouped_scale_split(const SplitJob *__restrict__ jobs, unsigned *status, unsigne
 // us, 64 columns 269 -> 187.  The planes' loads alone take 145 and 130 (0.6
 // GB each from HBM), the stores 30; the third stage is worth 5.
 
+// The GEMM kernels of a run do not depend on one another: each lets the next one's
+// blocks fill the SMs that its own last tiles leave idle (programmatic dependent
+// launch; 1187 -> 1171 us for 2304 problems), and ends after the kernel before it,
+// so that what follows the run follows all of them.
+__device__ __forceinline__ void end_beside() {
+  if (blockIdx.x == gridDim.x - 1) tc::griddep_wait();
+}
+
 // K slabs of a CTA's tile i (0 from `mine` on).
 __device__ __forceinline__ int tile_slabs(const Prob *probs, const Tile *tiles, int i, int mine) {
   if (i >= mine) return 0;
@@ -204,6 +213,7 @@ grouped_split_gemm(const CUtensorMap *__restrict__ tmaps, const Prob *__restrict
   uint64_t *turn = drain + 1;        // per accumulator group: its tile's last chunk is drained
   uint32_t *tmem_slot = (uint32_t *)(turn + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  tc::griddep_launch_dependents();
 
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; b++) tc::mbar_init(tc::smem_u32(&turn[b]), C_::GROUP_WARPS);
@@ -444,6 +454,7 @@ grouped_split_gemm(const CUtensorMap *__restrict__ tmaps, const Prob *__restrict
     tc::tc_fence_after();
     tc::tmem_dealloc(tmem, 512);
   }
+  end_beside();
 }
 
 // ---- split-K: ordered reduction of the slices ---------------------------------
@@ -481,8 +492,133 @@ grouped_splitk_reduce(const Prob *__restrict__ probs, const int *__restrict__ pr
   *dst = acc;
 }
 
-// ---- grouped CUDA-core kernel ---------------------------------------------------
+// ---- grouped CUDA-core kernels --------------------------------------------------
 
+__device__ __forceinline__ Gemm gemm_of(const Prob &P) {
+  Gemm g;
+  g.a = P.A; g.b = P.B; g.c = P.C;
+  g.M = P.M; g.K = P.K; g.N = P.N;
+  g.rsa = P.rsa; g.csa = P.csa; g.rsb = P.rsb; g.csb = P.csb; g.rso = P.rso; g.cso = P.cso;
+  g.isa = P.isa;
+  return g;
+}
+
+// The single-problem kernels' tiles (f32_tiles.cuh), one list entry a block: 16 x
+// 16 or 32 x 32 outputs (Tile::ks), copied 16 bytes at a time where the problem's
+// strides and alignment allow; SMALL: numc's unpacked path, 16 x 16.
+using Tile16 = f32::F32SmallCfg<8, 8, 2, 2>;
+using Tile32 = f32::F32SmallCfg<8, 8, 4, 4>;
+
+template <int T, bool SMALL>
+__device__ __forceinline__ void small_tile(const Gemm &g, const Tile &tl, float *smem) {
+  constexpr int Q = T / 8;
+  const bool va = f32::vec_a(g.a, g.rsa, g.csa), vb = f32::vec_b(g.b, g.rsb, g.csb);
+  if (va && vb) f32::f32_small_tile<8, 8, Q, Q, SMALL, true, true>(g, tl.m0, tl.n0, smem);
+  else if (va) f32::f32_small_tile<8, 8, Q, Q, SMALL, true, false>(g, tl.m0, tl.n0, smem);
+  else if (vb) f32::f32_small_tile<8, 8, Q, Q, SMALL, false, true>(g, tl.m0, tl.n0, smem);
+  else f32::f32_small_tile<8, 8, Q, Q, SMALL, false, false>(g, tl.m0, tl.n0, smem);
+}
+
+template <bool SMALL>
+__global__ void __launch_bounds__(64, 6)
+grouped_f32_small(const Prob *__restrict__ probs, const Tile *__restrict__ tiles) {
+  extern __shared__ __align__(16) float smem[];
+  const Tile tl = tiles[blockIdx.x];
+  const Gemm g = gemm_of(probs[tl.prob]);
+  tc::griddep_launch_dependents();
+  if (tl.ks == 16) small_tile<16, SMALL>(g, tl, smem);
+  else small_tile<32, SMALL>(g, tl, smem);
+  end_beside();
+}
+
+// 128 x 64 outputs, a block walking its share of the list: the first slabs of the
+// next tile are on their way while a tile is finished and stored, and the list
+// entries of later tiles while this one is computed; of a last slab only the
+// steps below K are multiplied.  Measured, us with 128 x 128 tiles of scalar FMAs
+// and a pass for the remainders before, and with these tiles and the 16 x 16 and 32 x
+// 32 ones now: plans of the plain algorithm, 64 problems of 16 to 1024 399 / 93,
+// 500 of 16 to 256 171 / 139, 16 of 512 to 2048 1597 / 1169, one of 2000^3 671 /
+// 424, 8 of 100 to 200 37 / 13.5; the 573 small problems of a mixed plan (most K
+// below 64: instructions of start and store weigh as much as the FMAs) 361 / 327.
+using TileBig = f32::F32Cfg<16, 8, 8, 8>;
+constexpr int kBigCtas = 3, kBigRing = 8;
+
+struct alignas(16) F32Job {
+  const float *A, *B;
+  float *C;
+  int64_t rsa, csa, rsb, csb, rso, cso;
+  int M, N, K, isa, m0, n0;
+};
+constexpr int kBigSmem = TileBig::SMEM + kBigRing * (int)sizeof(F32Job);
+
+__global__ void __launch_bounds__(128, kBigCtas)
+grouped_f32(const F32Job *__restrict__ jobs, int njobs) {
+  constexpr int BK = TileBig::BK, BM = TileBig::BM, BN = TileBig::BN, STAGES = TileBig::STAGES;
+  extern __shared__ __align__(16) float smem[];
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+  float *const edge_sums = smem + STAGES * TileBig::STAGE, *const bsum = edge_sums + threadIdx.x;
+  F32Job *const ring = reinterpret_cast<F32Job *>(smem + TileBig::SMEM / 4);
+  const int mine = (njobs - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
+  auto fetch_job = [&](int i) {   // this block's tile i to ring[i % kBigRing]
+    if (i < mine && threadIdx.x < sizeof(F32Job) / 16)
+      copy_async<16>(reinterpret_cast<float *>(ring + i % kBigRing) + 4 * threadIdx.x,
+                     reinterpret_cast<const float *>(jobs + blockIdx.x + (int64_t)i * gridDim.x) +
+                         4 * threadIdx.x);
+  };
+  f32::F32Loads<16, 8, 8, 8> ld;
+  f32::F32Acc<16, 8, 8, 8> acc;
+  auto first = [](int t, int n, int b) { return max(0, min(t, n - b)); };
+  int li = -1, left = 0, into = 0;   // tile being loaded, its k steps left, its next stage
+  auto load = [&] {   // the next slab of the block's tiles, if any
+    if (left <= 0 && li + 1 < mine) {
+      // its entry came with a group that is complete: three tiles, so at least
+      // three of these calls, ago (every tile has a slab)
+      const F32Job &J = ring[++li % kBigRing];
+      fetch_job(li + 3);
+      left = J.K;
+      ld.start(J.A, J.B, J.rsa, J.csa, J.rsb, J.csb, J.M, J.N, first(J.m0, J.M, BM),
+               first(J.n0, J.N, BN));
+    }
+    if (left > 0) {
+      ld.slab(sbase + into * TileBig::STAGE * 4, left);
+      left -= BK;
+      if (++into == STAGES) into = 0;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  tc::griddep_launch_dependents();
+  for (int i = 0; i < 3; i++) fetch_job(i);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+#pragma unroll 1
+  for (int t = 0; t < STAGES - 1; t++) load();
+  int stage = 0;
+  for (int i = 0; i < mine; i++) {
+    const F32Job &J = ring[i % kBigRing];
+    const int m0 = first(J.m0, J.M, BM), n0 = first(J.n0, J.N, BN);
+    const int slabs = (J.K + BK - 1) / BK;
+    acc.start(J.M, J.N, J.K, J.isa, m0, n0);
+    for (int t = 0; t < slabs; t++) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+      __syncthreads();   // slab t has arrived, and everyone is done with the one before
+      load();
+      if ((t + 1) * BK <= J.K) acc.slab(smem + stage * TileBig::STAGE);
+      else acc.part_slab(smem + stage * TileBig::STAGE, J.K - t * BK);
+      if (++stage == STAGES) stage = 0;
+      acc.end_slab(t, slabs, bsum);
+    }
+    acc.to_shared(edge_sums, bsum);
+    Gemm g;
+    g.c = J.C;
+    g.M = J.M; g.N = J.N;
+    g.rso = J.rso; g.cso = J.cso;
+    f32::store_tile<BM, BN, 128>(g, edge_sums, m0, n0, J.m0 - m0, J.n0 - n0);
+    __syncthreads();   // the stores' reads, before the next tile's edge sums
+  }
+  end_beside();
+}
+
+// Strides or K beyond 32-bit offsets: the general tile.
 constexpr int kSimtBM = 128, kSimtBN = 128;
 
 // numc_matmul's gemmsup threshold for float32 (src/matmul/matmul.c:241-256).
@@ -497,11 +633,7 @@ __global__ void __launch_bounds__(simt::kThreads, 2)
 grouped_simt(const Prob *__restrict__ probs, const Tile *__restrict__ tiles) {
   const Tile tl = tiles[blockIdx.x];
   const Prob &P = probs[tl.prob];
-  Gemm g;
-  g.a = P.A; g.b = P.B; g.c = P.C;
-  g.M = P.M; g.K = P.K; g.N = P.N;
-  g.rsa = P.rsa; g.csa = P.csa; g.rsb = P.rsb; g.csb = P.csb; g.rso = P.rso; g.cso = P.cso;
-  g.isa = P.isa;
+  const Gemm g = gemm_of(P);
   simt::simt_tile<float, kSimtBM, kSimtBN, 8, 8, 8, KIND>(g, 0, tl.m0, tl.n0);
 }
 
@@ -513,11 +645,7 @@ grouped_float_edges(const Prob *__restrict__ probs, const int *__restrict__ prob
                     const int2 *__restrict__ jobs) {
   const int2 job = jobs[blockIdx.x];
   const Prob &P = probs[probs_idx[job.x]];
-  Gemm g;
-  g.a = P.A; g.b = P.B; g.c = P.C;
-  g.M = P.M; g.K = P.K; g.N = P.N;
-  g.rsa = P.rsa; g.csa = P.csa; g.rsb = P.rsb; g.csb = P.csb; g.rso = P.rso; g.cso = P.cso;
-  g.isa = P.isa;
+  const Gemm g = gemm_of(P);
   const int64_t r0 = simt::edge_row<float>(g.M, g.isa), c0 = simt::edge_col<float>(g.N, g.isa);
   const int64_t n = simt::float_edge_groups<float>(g.M, g.N, g.isa);
   const int64_t gi = (int64_t)job.y * 16 + threadIdx.x / 16;
@@ -533,6 +661,9 @@ using namespace numc_k;
 using namespace numc_k::grouped;
 
 enum Variant : int { kVarTc128 = 0, kVarTc64 = 1, kVarSimt = 2, kNumVar = 3 };
+// Tile lists: one per tensor-core variant; the CUDA-core problems' by kernel
+// (kListWide: strides beyond 32-bit offsets).
+enum List : int { kListWide = kVarSimt, kListBig, kListSmall, kListUnpacked, kNumList };
 
 struct NumcCudaGemmPlan {
   int device;
@@ -548,19 +679,20 @@ struct NumcCudaGemmPlan {
   long long split_jobs;
   bool f16;                       // scaled float16 planes (else bfloat16)
   int2 *d_max_jobs;               // (problem, job) of each scale block (float16 planes)
+  F32Job *d_f32_jobs;             // kListBig's tiles
   SplitJob *d_fused_jobs;         // the blocks of the fused scale + split pass
   long long fused_jobs;
   long long max_jobs;
   int n_split_probs;
   Prob *d_split_probs;
-  Tile *d_tiles[kNumVar];
-  int ntiles[kNumVar];
-  int nsimt_packed;               // CUDA-core tiles of numc's packed path (listed first)
+  Tile *d_tiles[kNumList];
+  int ntiles[kNumList];
+  int nwide_packed;               // kListWide's tiles of numc's packed path (listed first)
   int *d_sk_probs;                // split-K problems (indices into probs)
   int2 *d_sk_jobs;                // (split-K problem, block) of each reduction block
   int n_sk_probs;
   long long sk_jobs;
-  int *d_edge_probs;              // CUDA-core problems with packed-path remainders
+  int *d_edge_probs;              // kListWide's problems with packed-path remainders
   int2 *d_edge_jobs;              // (edge problem, block) of each remainder block
   int n_edge_probs;
   long long edge_jobs;
@@ -650,6 +782,42 @@ int pick_splits(size_t M, size_t N, size_t K, int num_kb) {
   return std::max(1, std::min(sp, num_kb));
 }
 
+// Tile edge of every CUDA-core problem (128: 128 x 64; 0: strides beyond 32-bit
+// offsets).  A tile takes an SM `each` cycles a k next to others and `one` alone
+// (measured, gemm_f32.cu), and `fixed` cycles for its start and stores (2586 tiles
+// of 32 x 32 and K of 16 to 80 in 60 us, 7757 of 128 x 64 in 250).
+// The cheapest tile wins among those that are done, alone, before the device
+// has worked off the whole plan: few or deep problems take the small ones.
+std::vector<int> pick_f32_tiles(const NumcCudaGemmPlan *p) {
+  static constexpr struct { int bm, bn; double one, each, fixed; } kTiles[] = {
+      {16, 16, 20, 8.5, 2000}, {32, 32, 42, 20, 2500}, {128, 64, 129, 105, 4900}};
+  auto cost = [](const Prob &P, int t) {
+    return (kTiles[t].each * P.K + kTiles[t].fixed) *
+           ((P.M + kTiles[t].bm - 1) / kTiles[t].bm) * ((P.N + kTiles[t].bn - 1) / kTiles[t].bn);
+  };
+  // the tiles a problem can have: numc's unpacked path has no 128 x 64
+  auto kinds = [](const Prob &P) { return numc_packed(P) ? 3 : 2; };   // (nor K = 0)
+  std::vector<int> tile(p->probs.size(), 0);
+  double all = 0;
+  for (size_t i = 0; i < tile.size(); i++) {
+    const Prob &P = p->probs[i];
+    if (p->variant[i] != kVarSimt || !f32::fits(P.rsa, P.csa, P.rsb, P.csb, P.K)) continue;
+    tile[i] = 16;
+    double c = cost(P, 0);
+    for (int t = 1; t < kinds(P); t++) c = std::min(c, cost(P, t));
+    all += c / p->sms;
+  }
+  for (size_t i = 0; i < tile.size(); i++) {
+    const Prob &P = p->probs[i];
+    if (!tile[i]) continue;
+    int best = 0;
+    for (int t = 1; t < kinds(P); t++)
+      if (kTiles[t].one * P.K <= all && cost(P, t) < cost(P, best)) best = t;
+    tile[i] = kTiles[best].bm;
+  }
+  return tile;
+}
+
 int fail(cudaError_t e, const char *what) {
   cudaGetLastError();
   return NUMC_SET_ERROR(e == cudaErrorMemoryAllocation ? NUMC_ERR_MALLOC : NUMC_ERR_INTERNAL,
@@ -674,14 +842,30 @@ cudaError_t prepare_tc() {
                               Cfg<BN, STAGES, FLUSH>::SMEM);
 }
 
+// A launch that may run beside the kernel before it (end_beside), if there is one.
+template <class... P, class... Q>
+cudaError_t launch_beside(bool beside, void (*kern)(P...), int grid, int threads, int smem,
+                          cudaStream_t s, Q... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = beside && pdl_enabled() ? 1 : 0;
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, (P)args...);
+}
+
 template <int BN, int STAGES, int FLUSH, bool F16>
-cudaError_t launch_tc(const NumcCudaGemmPlan *p, int var, unsigned *status, cudaStream_t s) {
+cudaError_t launch_tc(bool beside, const NumcCudaGemmPlan *p, int var, unsigned *status,
+                      cudaStream_t s) {
   using C_ = Cfg<BN, STAGES, FLUSH>;
-  auto kern = grouped_split_gemm<BN, STAGES, FLUSH, F16>;
-  const int grid = std::min(p->ntiles[var], p->sms);
-  kern<<<grid, C_::THREADS, C_::SMEM, s>>>(p->d_tmaps, p->d_probs, p->d_tiles[var],
-                                          p->ntiles[var], status, p->gen, wait_cfg());
-  return cudaGetLastError();
+  return launch_beside(beside, grouped_split_gemm<BN, STAGES, FLUSH, F16>,
+                       std::min(p->ntiles[var], p->sms), C_::THREADS, C_::SMEM, s, p->d_tmaps,
+                       p->d_probs, p->d_tiles[var], p->ntiles[var], status, p->gen, wait_cfg());
 }
 
 // Enqueue one run; `kernels` receives the number of kernels launched.
@@ -713,16 +897,40 @@ int plan_enqueue(NumcCudaGemmPlan *p, cudaStream_t s, unsigned *kernels) {
     if ((e = cudaGetLastError())) return fail(e, "grouped split");
     ++*kernels;
   }
+  bool beside = false;   // the first of these waits for the planes
   if (p->ntiles[kVarTc128]) {
-    e = p->f16 ? launch_tc<128, 3, kFlushF16, true>(p, kVarTc128, status, s)
-               : launch_tc<128, 3, kFlushBf16, false>(p, kVarTc128, status, s);
+    e = p->f16 ? launch_tc<128, 3, kFlushF16, true>(beside, p, kVarTc128, status, s)
+               : launch_tc<128, 3, kFlushBf16, false>(beside, p, kVarTc128, status, s);
     if (e) return fail(e, "grouped split GEMM (128)");
     ++*kernels;
+    beside = true;
   }
   if (p->ntiles[kVarTc64]) {
-    e = p->f16 ? launch_tc<64, 4, kFlushF16, true>(p, kVarTc64, status, s)
-               : launch_tc<64, 4, kFlushBf16, false>(p, kVarTc64, status, s);
+    e = p->f16 ? launch_tc<64, 4, kFlushF16, true>(beside, p, kVarTc64, status, s)
+               : launch_tc<64, 4, kFlushBf16, false>(beside, p, kVarTc64, status, s);
     if (e) return fail(e, "grouped split GEMM (64)");
+    ++*kernels;
+    beside = true;
+  }
+  if (p->ntiles[kListBig]) {
+    e = launch_beside(beside, grouped_f32, std::min(p->ntiles[kListBig], kBigCtas * p->sms), 128,
+                      kBigSmem, s, p->d_f32_jobs, p->ntiles[kListBig]);
+    if (e) return fail(e, "grouped float32 (128 x 64)");
+    ++*kernels;
+    beside = true;
+  }
+  constexpr int small_smem = std::max(Tile16::SMEM, Tile32::SMEM);
+  if (p->ntiles[kListUnpacked]) {
+    e = launch_beside(beside, grouped_f32_small<true>, p->ntiles[kListUnpacked], 64, small_smem, s,
+                      p->d_probs, p->d_tiles[kListUnpacked]);
+    if (e) return fail(e, "grouped float32 (unpacked path)");
+    ++*kernels;
+    beside = true;
+  }
+  if (p->ntiles[kListSmall]) {
+    e = launch_beside(beside, grouped_f32_small<false>, p->ntiles[kListSmall], 64, small_smem, s,
+                      p->d_probs, p->d_tiles[kListSmall]);
+    if (e) return fail(e, "grouped float32");
     ++*kernels;
   }
   if (p->sk_jobs > 0) {
@@ -735,15 +943,15 @@ int plan_enqueue(NumcCudaGemmPlan *p, cudaStream_t s, unsigned *kernels) {
     if ((e = cudaGetLastError())) return fail(e, "grouped split-K reduction");
     ++*kernels;
   }
-  if (p->nsimt_packed) {
-    grouped_simt<simt::kFloat><<<p->nsimt_packed, simt::kThreads, 0, s>>>(
-        p->d_probs, p->d_tiles[kVarSimt]);
+  if (p->nwide_packed) {
+    grouped_simt<simt::kFloat><<<p->nwide_packed, simt::kThreads, 0, s>>>(
+        p->d_probs, p->d_tiles[kListWide]);
     if ((e = cudaGetLastError())) return fail(e, "grouped SIMT");
     ++*kernels;
   }
-  if (p->ntiles[kVarSimt] > p->nsimt_packed) {
-    grouped_simt<simt::kFloatSmall><<<p->ntiles[kVarSimt] - p->nsimt_packed, simt::kThreads, 0,
-                                      s>>>(p->d_probs, p->d_tiles[kVarSimt] + p->nsimt_packed);
+  if (p->ntiles[kListWide] > p->nwide_packed) {
+    grouped_simt<simt::kFloatSmall><<<p->ntiles[kListWide] - p->nwide_packed, simt::kThreads, 0,
+                                      s>>>(p->d_probs, p->d_tiles[kListWide] + p->nwide_packed);
     if ((e = cudaGetLastError())) return fail(e, "grouped SIMT (unpacked path)");
     ++*kernels;
   }
@@ -857,27 +1065,39 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) {
     return p->probs[x].num_kb / p->probs[x].splits > p->probs[y].num_kb / p->probs[y].splits;
   });
-  std::vector<Tile> tiles[kNumVar], simt_small;
+  std::vector<Tile> tiles[kNumList], wide_unpacked;
   std::vector<size_t> split_idx;
   std::vector<int> edge_idx;
+  const std::vector<int> f32_tile = pick_f32_tiles(p);
   for (size_t i : order) {
     const int v = p->variant[i];
     if (v < 0) continue;
-    if (v == kVarSimt && simt::float_edges_needed<float>(p->probs[i].K) && numc_packed(p->probs[i]) &&
-        simt::float_edge_count<float>(p->probs[i].M, p->probs[i].N, p->probs[i].isa) > 0)
-      edge_idx.push_back((int)i);
-    const int bn = v == kVarTc128 ? 128 : v == kVarTc64 ? 64 : kSimtBN;
-    const int bm = v == kVarSimt ? kSimtBM : kBM;
-    // CUDA-core problems on numc's unpacked path go to a list of their own
-    std::vector<Tile> &tl = (v == kVarSimt && !numc_packed(p->probs[i])) ? simt_small : tiles[v];
-    for (int m0 = 0; m0 < p->probs[i].M; m0 += bm)
-      for (int n0 = 0; n0 < p->probs[i].N; n0 += bn)
-        for (int ks = 0; ks < p->probs[i].splits; ks++) tl.push_back(Tile{(int)i, m0, n0, ks});
-    if (v != kVarSimt) split_idx.push_back(i);
+    const Prob &P = p->probs[i];
+    int bm = kBM, bn = v == kVarTc128 ? 128 : 64, list = v;
+    if (v != kVarSimt) {
+      split_idx.push_back(i);
+    } else if (f32_tile[i] == 128) {
+      list = kListBig;   // 128 x 64
+    } else if (f32_tile[i]) {
+      bm = bn = f32_tile[i];
+      list = numc_packed(P) ? kListSmall : kListUnpacked;
+    } else {
+      bm = kSimtBM, bn = kSimtBN;
+      if (simt::float_edges_needed<float>(P.K) && numc_packed(P) &&
+          simt::float_edge_count<float>(P.M, P.N, P.isa) > 0)
+        edge_idx.push_back((int)i);
+    }
+    std::vector<Tile> &tl = list == kListWide && !numc_packed(P) ? wide_unpacked : tiles[list];
+    for (int m0 = 0; m0 < P.M; m0 += bm)
+      for (int n0 = 0; n0 < P.N; n0 += bn)
+        if (v == kVarSimt)
+          tl.push_back(Tile{(int)i, m0, n0, bm});
+        else
+          for (int ks = 0; ks < P.splits; ks++) tl.push_back(Tile{(int)i, m0, n0, ks});
   }
-  // the CUDA-core list: numc's packed-path problems, then the unpacked ones
-  p->nsimt_packed = (int)tiles[kVarSimt].size();
-  tiles[kVarSimt].insert(tiles[kVarSimt].end(), simt_small.begin(), simt_small.end());
+  // the wide-stride list: numc's packed-path problems, then the unpacked ones
+  p->nwide_packed = (int)tiles[kListWide].size();
+  tiles[kListWide].insert(tiles[kListWide].end(), wide_unpacked.begin(), wide_unpacked.end());
   // Job tables: (problem, job within it) for every block of the scale,
   // split and remainder passes, so a block finds its problem in one load.
   std::vector<int2> split_jobs, max_jobs, edge_jobs;
@@ -942,12 +1162,13 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   const size_t o_split_jobs = off; off = align_up(off + split_jobs.size() * sizeof(int2), 256);
   const size_t o_max_jobs = off; off = align_up(off + max_jobs.size() * sizeof(int2), 256);
   const size_t o_fused_jobs = off; off = align_up(off + (size_t)n_fused * sizeof(SplitJob), 256);
+  const size_t o_f32 = off; off = align_up(off + tiles[kListBig].size() * sizeof(F32Job), 256);
   const size_t o_sk = off; off = align_up(off + sk_idx.size() * sizeof(int), 256);
   const size_t o_sk_jobs = off; off = align_up(off + sk_jobs.size() * sizeof(int2), 256);
   const size_t o_edges = off; off = align_up(off + edge_idx.size() * sizeof(int), 256);
   const size_t o_edge_jobs = off; off = align_up(off + edge_jobs.size() * sizeof(int2), 256);
-  size_t o_tiles[kNumVar];
-  for (int v = 0; v < kNumVar; v++) {
+  size_t o_tiles[kNumList];
+  for (int v = 0; v < kNumList; v++) {
     o_tiles[v] = off;
     off = align_up(off + tiles[v].size() * sizeof(Tile), 256);
   }
@@ -967,12 +1188,13 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   p->d_split_jobs = (int2 *)(p->dev + o_split_jobs);
   p->d_max_jobs = (int2 *)(p->dev + o_max_jobs);
   p->d_fused_jobs = (SplitJob *)(p->dev + o_fused_jobs);
+  p->d_f32_jobs = (F32Job *)(p->dev + o_f32);
   p->d_sk_probs = (int *)(p->dev + o_sk);
   p->d_sk_jobs = (int2 *)(p->dev + o_sk_jobs);
   p->d_edge_probs = (int *)(p->dev + o_edges);
   p->d_edge_jobs = (int2 *)(p->dev + o_edge_jobs);
   p->n_edge_probs = (int)edge_idx.size();
-  for (int v = 0; v < kNumVar; v++) {
+  for (int v = 0; v < kNumList; v++) {
     p->d_tiles[v] = (Tile *)(p->dev + o_tiles[v]);
     p->ntiles[v] = (int)tiles[v].size();
   }
@@ -1007,6 +1229,8 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   // Kernel attributes are set here, not per run, so runs can be captured.
   if ((e = prepare_tc<128, 3, kFlushBf16, false>()) || (e = prepare_tc<64, 4, kFlushBf16, false>()) ||
       (e = prepare_tc<128, 3, kFlushF16, true>()) || (e = prepare_tc<64, 4, kFlushF16, true>()) ||
+      (e = cudaFuncSetAttribute(grouped_f32, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kBigSmem)) ||
       !status_word()) {
     numc_cuda_gemm_plan_free(p);
     fail(e ? e : cudaErrorMemoryAllocation, "plan kernel setup");
@@ -1050,8 +1274,21 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
     fail(e, "plan upload");
     return nullptr;
   }
-  for (int v = 0; v < kNumVar; v++)
-    if (!tiles[v].empty() &&
+  std::vector<F32Job> fj;
+  fj.reserve(tiles[kListBig].size());
+  for (const Tile &t : tiles[kListBig]) {
+    const Prob &P = p->probs[t.prob];
+    fj.push_back(F32Job{P.A, P.B, P.C, P.rsa, P.csa, P.rsb, P.csb, P.rso, P.cso, P.M, P.N, P.K,
+                        P.isa, t.m0, t.n0});
+  }
+  if (!fj.empty() && (e = cudaMemcpy(p->d_f32_jobs, fj.data(), fj.size() * sizeof(F32Job),
+                                     cudaMemcpyHostToDevice))) {
+    numc_cuda_gemm_plan_free(p);
+    fail(e, "plan upload");
+    return nullptr;
+  }
+  for (int v = 0; v < kNumList; v++)
+    if (v != kListBig && !tiles[v].empty() &&
         (e = cudaMemcpy(p->d_tiles[v], tiles[v].data(), tiles[v].size() * sizeof(Tile),
                         cudaMemcpyHostToDevice))) {
       numc_cuda_gemm_plan_free(p);
