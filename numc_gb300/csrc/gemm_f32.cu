@@ -118,12 +118,13 @@ bool launch_f32_packed(const Gemm &g, cudaStream_t s, cudaError_t *e) {
   // Tiles, and measured cycles per k of one CTA alone on an SM and of each of
   // several (GB300, 64 x 1000 x 64 to 8192^3), for operands that the small
   // kernel can copy 16 bytes at a time and for others: the K loop of an SM's
-  // CTAs decides, so the tile whose count rounds best wins.
+  // CTAs decides, so the tile whose count rounds best wins (500 x 1000 x 450, two
+  // 32 x 32 tiles an SM: 43 us with the small kernel, 33 with the packed one).
   static constexpr struct { int bm, bn; double one[2], each[2]; } kTiles[] = {
       {128, 96, {166, 166}, {140, 140}}, {128, 80, {143, 143}, {124, 124}},
       {128, 64, {129, 129}, {105, 105}}, {64, 64, {118, 118}, {62, 62}},
       {32, 64, {75, 75}, {38, 38}},      {32, 32, {47, 47}, {22, 22}},
-      {32, 32, {38, 46}, {18, 23}},      {16, 16, {17, 23}, {8, 9}}};
+      {32, 32, {38, 64}, {18, 42}},      {16, 16, {17, 23}, {8, 9}}};
   const int odd = !(vec_a(g.a, g.rsa, g.csa) && vec_b(g.b, g.rsb, g.csb));
   const int64_t sms = sm_count();
   int best = 0;

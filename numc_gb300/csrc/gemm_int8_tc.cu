@@ -926,7 +926,7 @@ cudaError_t launch_i8(const Gemm &g, int rule, int tile, char *ws, const I8Layou
   int bn = tile == kI8TilePair128 ? 128 : 256;
   if (tile == kI8TileAuto) {
     tile = pick_tile(g);
-    bn = pair_tile_columns(g.M, g.N);
+    bn = pair_tile_columns(g.M, g.N, g.K);
   }
   if (tile == kI8TilePair256)
     e = x86 ? launch_i8_pair<SIGNED, 256, true>(g, rule, L, pa, pb, bn, status, s)

@@ -66,13 +66,15 @@ int sm_count() {
   return cached[dev];
 }
 
-int pair_tile_columns(int64_t M, int64_t N) {
+int pair_tile_columns(int64_t M, int64_t N, int64_t K) {
   const int64_t pairs = std::max(1, sm_count() / 2), tm = (M + 255) / 256;
   int best = 256;
   int64_t t_best = 0;
   for (int bn = 256; bn >= 160; bn -= 32) {
     const int64_t rounds = (tm * ((N + bn - 1) / bn) + pairs - 1) / pairs;
-    const int64_t t = rounds * (bn + 16);   // 16: a tile's own start and end
+    // 64 for the A operand's share, and a tile's start and end, which weigh the
+    // more the fewer 64-deep slabs it has
+    const int64_t t = rounds * (bn + 64 + 128 * 64 / std::max<int64_t>(K, 64));
     if (bn == 256 || t < t_best) {
       best = bn;
       t_best = t;
@@ -926,10 +928,13 @@ int forced_tile() {
 // Columns of the CTA pairs' wide tiles, 256 or a little less: the width whose
 // rounds of tiles over the pairs multiply the fewest columns (the last round of
 // 256-column tiles may occupy few pairs: 4096^2 is 3.4 rounds of them, 4.0 of 224
-// columns; GEMM 261 -> 240 us).
+// columns; GEMM 261 -> 240 us).  Narrower tiles read A more often and shallow ones
+// are mostly start and end: 192 instead of 256 columns took 2537 x 153 x 6853 from
+// 43.8 to 46.2 us, 6578 x 3956 x 2560 from 298 to 301, and 224 instead of 256 7000 x
+// 128 x 7000 from 89.9 to 92.4, so those keep 256.
 int wide_tile_columns(const Gemm &g) {
   if (forced_tile()) return 256;
-  return pair_tile_columns(g.M, g.N);
+  return pair_tile_columns(g.M, g.N, g.K);
 }
 
 template <int BN, int STAGES, int PLANES, int FLUSH, bool F16, int CTAS>

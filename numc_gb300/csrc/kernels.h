@@ -179,7 +179,7 @@ cudaError_t dev_malloc(void **p, size_t bytes);
 int sm_count();
 // Columns (160 to 256) of 256-row tiles on CTA pairs that round an M x N output
 // best over the device's pairs.
-int pair_tile_columns(int64_t M, int64_t N);
+int pair_tile_columns(int64_t M, int64_t N, int64_t K);
 // Programmatic dependent launch of GEMM kernels after their operand passes
 // (on unless the environment sets NUMC_CUDA_PDL=0).
 bool pdl_enabled();
