@@ -135,7 +135,7 @@ NUMC_API NumcArray *numc_cuda_array_rand(NumcCtx *ctx, const size_t *shape,
                                          size_t dim, NumcDType dtype);
 /* numc_array_rand's fill of n elements of `dtype` at device pointer `out`,
  * enqueued on `stream` (a cudaStream_t); advances the calling thread's
- * state.  The first fill on a device uploads the generator's 1 MiB jump
+ * state.  The first fill on a device uploads the generator's 0.9 MiB jump
  * tables there (cudaMalloc, kept until exit). */
 NUMC_API int numc_cuda_rand_fill(NumcDType dtype, void *out, size_t n,
                                  void *stream);
@@ -147,7 +147,9 @@ NUMC_API int numc_cuda_rand_threads(void);
 
 /* --- C-ABI GEMM on device pointers -------------------------------------- */
 
-/* Scratch bytes numc_cuda_gemm needs for this problem (0 for SIMT/DMMA). */
+/* Scratch bytes numc_cuda_gemm needs for this problem (0 for SIMT/DMMA).
+ * 16- to 64-bit integers with NUMC_CUDA_ALGO_DEFAULT: the digit planes of the
+ * tensor-core path where that is the faster one, else 0. */
 NUMC_API size_t numc_cuda_gemm_workspace_size(NumcDType dtype, int algo,
                                               int param, size_t M, size_t K,
                                               size_t N);
@@ -156,7 +158,8 @@ NUMC_API size_t numc_cuda_gemm_workspace_size(NumcDType dtype, int algo,
  * arithmetic for `dtype`.  a, b, out are device pointers; strides are in
  * elements.  `workspace` may be NULL (the library then keeps a per-device
  * scratch buffer, grown with cudaMalloc) or caller memory of at least
- * numc_cuda_gemm_workspace_size() bytes, aligned to 256 bytes.  `stream` is
+ * numc_cuda_gemm_workspace_size() bytes, aligned to 256 bytes.  16- to 64-bit
+ * integers without such a workspace run on the CUDA cores (same results).  `stream` is
  * a cudaStream_t (NULL = legacy default stream).  Asynchronous: returns
  * after enqueueing; launch errors are returned, kernel-side timeouts are
  * reported by numc_cuda_check_status(). */

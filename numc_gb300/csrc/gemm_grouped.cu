@@ -9,10 +9,10 @@
 // uploads per-variant tile lists.  Running it enqueues only:
 //   1. a memset of the non-finite flags (and row / column maxima),
 //   2. for scaled float16 planes (NUMC_CUDA_ALGO_SPLIT_FP16, the default),
-//      one grouped scale pass: row maxima of every A, column maxima of
-//      every B,
-//   3. one grouped split pass over every tensor-core problem (x -> two
-//      16-bit planes; a block reads its problem from a job table),
+//      one grouped pass over every tensor-core problem: row maxima of A,
+//      column maxima of B, and both planes,
+//   3. for bfloat16 planes, one grouped split pass (x -> two 16-bit planes; a
+//      block reads its problem from a job table),
 //   4. one persistent split tcgen05 kernel per tile width (128 or 64
 //      columns): each CTA walks a static share of the variant's tile list;
 //      the TMA ring, the MMA chunk stream and the TMEM buffers run on
@@ -161,7 +161,7 @@ grouped_scale_split(const SplitJob *__restrict__ jobs, unsigned *status, unsigne
 // lane and the maxima loaded before the first chunk, 2304 problems of 16 to
 // 1024 (24 and 42 tiles a CTA; mostly 1 to 8 slabs): 128 columns 315 -> 211
 // us, 64 columns 269 -> 187.  The planes' loads alone take 145 and 130 (0.6
-// GB each from HBM), the stores 30; the third stage is worth 5.
+// GB each from HBM), the stores 36 and 10; the third stage is worth 5.
 
 // The GEMM kernels of a run do not depend on one another: each lets the next one's
 // blocks fill the SMs that its own last tiles leave idle (programmatic dependent
