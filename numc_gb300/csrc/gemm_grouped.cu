@@ -78,34 +78,10 @@ __host__ __device__ inline void slice_range(const Prob &P, int ks, int &kb0, int
   kb1 = (int)((int64_t)(ks + 1) * P.num_kb / P.splits);
 }
 
-// ---- grouped scale pass (float16 planes) -----------------------------------------
-
-// Block b handles scale job jobs[b] = (problem p, job j of p): the blocks of
-// absmax_grid(M, K) over A's rows, then those of absmax_grid(N, K) over B's
-// columns.
-__global__ void __launch_bounds__(256)
-grouped_absmax(const Prob *__restrict__ probs, const int2 *__restrict__ jobs) {
-  const int2 job = jobs[blockIdx.x];
-  const Prob &P = probs[job.x];
-  long long j = job.y;
-  const int ma = absmax_mode(P.split_mode_a, P.csa);
-  const dim3 ga = absmax_grid(P.M, P.K, ma);
-  const long long a_jobs = (long long)ga.x * ga.y;
-  if (j < a_jobs) {
-    absmax_block(P.A, P.rsa, P.csa, P.M, P.K, ma, P.max_a, j % ga.x, j / ga.x);
-  } else {
-    j -= a_jobs;
-    const int mb = absmax_mode(P.split_mode_b, P.rsb);
-    const dim3 gb = absmax_grid(P.N, P.K, mb);
-    absmax_block(P.B, P.csb, P.rsb, P.N, P.K, mb, P.max_b, j % gb.x, j / gb.x);
-  }
-}
-
 // ---- grouped split pass --------------------------------------------------------
 
 // Block b handles split job jobs[b] = (problem p, job j of p): A tiles
 // (ceil(M/32) x ceil(Kp/128)) come first, then B tiles.
-template <bool F16>
 __global__ void __launch_bounds__(256)
 grouped_split(const Prob *__restrict__ probs, const int2 *__restrict__ jobs,
               unsigned long long gen) {
@@ -116,12 +92,12 @@ grouped_split(const Prob *__restrict__ probs, const int2 *__restrict__ jobs,
   const long long kt = (P.Kp + kSplitK - 1) / kSplitK;
   const long long a_jobs = (long long)((P.M + kSplitRows - 1) / kSplitRows) * kt;
   if (j < a_jobs) {
-    split_tile<kPlanes, F16>(P.A, P.rsa, P.csa, P.M, P.K, P.Kp, P.pa, P.flags_a, kBM, gen,
+    split_tile<kPlanes, false>(P.A, P.rsa, P.csa, P.M, P.K, P.Kp, P.pa, P.flags_a, kBM, gen,
                              P.split_mode_a, (j / kt) * kSplitRows, (j % kt) * kSplitK, tile,
                              P.max_a);
   } else {
     j -= a_jobs;
-    split_tile<kPlanes, F16>(P.B, P.csb, P.rsb, P.N, P.K, P.Kp, P.pb, P.flags_b, 64, gen,
+    split_tile<kPlanes, false>(P.B, P.csb, P.rsb, P.N, P.K, P.Kp, P.pb, P.flags_b, 64, gen,
                              P.split_mode_b, (j / kt) * kSplitRows, (j % kt) * kSplitK, tile,
                              P.max_b);
   }
@@ -678,11 +654,9 @@ struct NumcCudaGemmPlan {
   int2 *d_split_jobs;             // (problem, job) of each split block
   long long split_jobs;
   bool f16;                       // scaled float16 planes (else bfloat16)
-  int2 *d_max_jobs;               // (problem, job) of each scale block (float16 planes)
   F32Job *d_f32_jobs;             // kListBig's tiles
   SplitJob *d_fused_jobs;         // the blocks of the fused scale + split pass
   long long fused_jobs;
-  long long max_jobs;
   int n_split_probs;
   Prob *d_split_probs;
   Tile *d_tiles[kNumList];
@@ -876,11 +850,6 @@ int plan_enqueue(NumcCudaGemmPlan *p, cudaStream_t s, unsigned *kernels) {
   cudaError_t e;
   if (p->flags_bytes && (e = cudaMemsetAsync(p->flags, 0, p->flags_bytes, s)))
     return fail(e, "plan flags");
-  if (p->f16 && p->max_jobs > 0) {
-    grouped_absmax<<<(unsigned)p->max_jobs, 256, 0, s>>>(p->d_split_probs, p->d_max_jobs);
-    if ((e = cudaGetLastError())) return fail(e, "grouped scale pass");
-    ++*kernels;
-  }
   if (p->fused_jobs > 0) {
     grouped_scale_split<<<(unsigned)p->fused_jobs, 256, 0, s>>>(p->d_fused_jobs, status, p->gen,
                                                                   wait_cfg());
@@ -888,12 +857,7 @@ int plan_enqueue(NumcCudaGemmPlan *p, cudaStream_t s, unsigned *kernels) {
     ++*kernels;
   }
   if (p->split_jobs > 0) {
-    if (p->f16)
-      grouped_split<true><<<(unsigned)p->split_jobs, 256, 0, s>>>(p->d_split_probs,
-                                                                  p->d_split_jobs, p->gen);
-    else
-      grouped_split<false><<<(unsigned)p->split_jobs, 256, 0, s>>>(p->d_split_probs,
-                                                                   p->d_split_jobs, p->gen);
+    grouped_split<<<(unsigned)p->split_jobs, 256, 0, s>>>(p->d_split_probs, p->d_split_jobs, p->gen);
     if ((e = cudaGetLastError())) return fail(e, "grouped split");
     ++*kernels;
   }
@@ -1100,7 +1064,7 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   tiles[kListWide].insert(tiles[kListWide].end(), wide_unpacked.begin(), wide_unpacked.end());
   // Job tables: (problem, job within it) for every block of the scale,
   // split and remainder passes, so a block finds its problem in one load.
-  std::vector<int2> split_jobs, max_jobs, edge_jobs;
+  std::vector<int2> split_jobs, edge_jobs;
   long long n_fused = 0;
   for (size_t q = 0; q < split_idx.size(); q++) {
     const Prob &P = p->probs[split_idx[q]];
@@ -1113,12 +1077,6 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
     const long long n = ((P.M + kSplitRows - 1) / kSplitRows) * kt +
                         ((P.N + kSplitRows - 1) / kSplitRows) * kt;
     for (long long j = 0; j < n; j++) split_jobs.push_back(make_int2((int)q, (int)j));
-    if (p->f16) {
-      const dim3 ga = absmax_grid(P.M, P.K, absmax_mode(P.split_mode_a, P.csa));
-      const dim3 gb = absmax_grid(P.N, P.K, absmax_mode(P.split_mode_b, P.rsb));
-      const long long nm = (long long)ga.x * ga.y + (long long)gb.x * gb.y;
-      for (long long j = 0; j < nm; j++) max_jobs.push_back(make_int2((int)q, (int)j));
-    }
   }
   // split-K problems: partial sums (splits x M x N floats each) and the
   // reduction's blocks
@@ -1142,12 +1100,11 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   }
   p->split_jobs = (long long)split_jobs.size();
   p->n_split_probs = (int)split_idx.size();
-  p->max_jobs = (long long)max_jobs.size();
   p->edge_jobs = (long long)edge_jobs.size();
   p->fused_jobs = n_fused;
   p->sk_jobs = (long long)sk_jobs.size();
   p->n_sk_probs = (int)sk_idx.size();
-  if (p->split_jobs > 0x7FFFFFFFll || p->max_jobs > 0x7FFFFFFFll || p->edge_jobs > 0x7FFFFFFFll ||
+  if (p->split_jobs > 0x7FFFFFFFll || p->edge_jobs > 0x7FFFFFFFll ||
       p->fused_jobs > 0x7FFFFFFFll || p->sk_jobs > 0x7FFFFFFFll) {
     delete p;
     NUMC_SET_ERROR(NUMC_ERR_VALUE, "plan_create: too many split blocks");
@@ -1160,7 +1117,6 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   const size_t o_probs = off; off = align_up(off + count * sizeof(Prob), 256);
   const size_t o_sprobs = off; off = align_up(off + split_idx.size() * sizeof(Prob), 256);
   const size_t o_split_jobs = off; off = align_up(off + split_jobs.size() * sizeof(int2), 256);
-  const size_t o_max_jobs = off; off = align_up(off + max_jobs.size() * sizeof(int2), 256);
   const size_t o_fused_jobs = off; off = align_up(off + (size_t)n_fused * sizeof(SplitJob), 256);
   const size_t o_f32 = off; off = align_up(off + tiles[kListBig].size() * sizeof(F32Job), 256);
   const size_t o_sk = off; off = align_up(off + sk_idx.size() * sizeof(int), 256);
@@ -1186,7 +1142,6 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
   p->d_probs = (Prob *)(p->dev + o_probs);
   p->d_split_probs = (Prob *)(p->dev + o_sprobs);
   p->d_split_jobs = (int2 *)(p->dev + o_split_jobs);
-  p->d_max_jobs = (int2 *)(p->dev + o_max_jobs);
   p->d_fused_jobs = (SplitJob *)(p->dev + o_fused_jobs);
   p->d_f32_jobs = (F32Job *)(p->dev + o_f32);
   p->d_sk_probs = (int *)(p->dev + o_sk);
@@ -1253,9 +1208,6 @@ extern "C" NumcCudaGemmPlan *numc_cuda_gemm_plan_create(NumcDType dtype, int alg
       (e = cudaMemcpy(p->d_split_probs, sp.data(), sp.size() * sizeof(Prob), cudaMemcpyHostToDevice)) ||
       (!split_jobs.empty() &&
        (e = cudaMemcpy(p->d_split_jobs, split_jobs.data(), split_jobs.size() * sizeof(int2),
-                       cudaMemcpyHostToDevice))) ||
-      (!max_jobs.empty() &&
-       (e = cudaMemcpy(p->d_max_jobs, max_jobs.data(), max_jobs.size() * sizeof(int2),
                        cudaMemcpyHostToDevice))) ||
       (!sj.empty() &&
        (e = cudaMemcpy(p->d_fused_jobs, sj.data(), sj.size() * sizeof(SplitJob),
