@@ -113,7 +113,13 @@ NUMC_API int numc_cuda_get_isa_profile(void);
 /* --- device residency --------------------------------------------------- */
 
 /* Copy the array to HBM and make the device copy authoritative: later
- * numc_matmul calls read/write it there without host transfers. */
+ * numc_matmul calls read/write it there without host transfers.  A 16- to
+ * 64-bit integer product (numc_matmul, numc_linear, numc_bmm, numc_dot) whose
+ * arrays are all resident is enqueued and returns, except that it waits for the
+ * context's earlier work when it needs more scratch than any call before it.
+ * Should its kernel abandon a bounded wait, the context's next
+ * numc_cuda_array_to_host, numc_cuda_ctx_synchronize or integer product with a
+ * host array, or numc_cuda_check_status, returns NUMC_ERR_INTERNAL. */
 NUMC_API int numc_cuda_array_to_device(NumcArray *arr);
 /* Copy a device-resident array back into its host buffer (it stays
  * resident; both copies are valid until the next device write). */

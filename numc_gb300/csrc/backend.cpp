@@ -309,8 +309,10 @@ size_t plan_workspace(NumcDType dt, const Plan &p, size_t M, size_t K, size_t N)
   return 0;
 }
 
+// `failure`: the word that the integer digit GEMM's kernels report in, the
+// device's status word if null.
 int run_plan(NumcDType dt, const Plan &p, const numc_k::Gemm &g, void *ws,
-             size_t ws_bytes, cudaStream_t s) {
+             size_t ws_bytes, cudaStream_t s, unsigned *failure = nullptr) {
   cudaError_t e = cudaSuccess;
   switch (p.algo) {
   case NUMC_CUDA_ALGO_SIMT: e = numc_k::launch_simt(dt, g, p.param, s); break;
@@ -319,7 +321,9 @@ int run_plan(NumcDType dt, const Plan &p, const numc_k::Gemm &g, void *ws,
   case NUMC_CUDA_ALGO_SPLIT_FP16: e = numc_k::launch_split_f16(g, p.param, ws, ws_bytes, s); break;
   case NUMC_CUDA_ALGO_OZAKI: e = numc_k::launch_ozaki(g, p.param, ws, ws_bytes, s); break;
   case NUMC_CUDA_ALGO_TC_INT8: e = numc_k::launch_int8_tc(dt, g, p.param, ws, ws_bytes, s); break;
-  case kAlgoIntDigits: e = numc_k::launch_int_digits(dt, g, ws, ws_bytes, s); break;
+  case kAlgoIntDigits:
+    e = numc_k::launch_int_digits(dt, g, ws, ws_bytes, failure ? failure : numc_k::status_word(), s);
+    break;
   }
   if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
   return 0;
@@ -366,10 +370,9 @@ int ctx_scratch(NumcCtx *ctx, size_t bytes, cudaStream_t s, char **out) {
 // Scratch of `base` bytes for staged operands plus the plan's workspace
 // (*ws_bytes).  Integer plans give the tensor cores up for the CUDA cores,
 // which need no workspace, where the device has no room for the digits, where
-// the stream is being captured (the call then neither allocates nor reads the
-// status word), and, with an asynchronous result (`async`: a resident output and
-// inputs), where they would not save more than the status word's read costs the
-// caller (about 15 us).
+// the stream is being captured (the digits would lie in scratch that a later call
+// may free), and, with an asynchronous result (`async`: a resident output and
+// inputs), where they would not save 15 us.
 int plan_scratch(NumcCtx *ctx, NumcDType dt, Plan *plan, size_t M, size_t K, size_t N,
                  size_t base, bool async, cudaStream_t s, size_t *ws_bytes, char **out) {
   *ws_bytes = plan_workspace(dt, *plan, M, K, N);
@@ -377,7 +380,8 @@ int plan_scratch(NumcCtx *ctx, NumcDType dt, Plan *plan, size_t M, size_t K, siz
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     const bool captured =
         cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
-    if (captured || (async && numc_k::int_digits_gain_us(dt, M, K, N) < 15) ||
+    if (!ctx->failure && !captured) ctx->failure = numc_k::failure_word_alloc();
+    if (captured || !ctx->failure || (async && numc_k::int_digits_gain_us(dt, M, K, N) < 15) ||
         grow_scratch(ctx, base + *ws_bytes + 256, s) != cudaSuccess) {
       cudaGetLastError();
       plan->algo = NUMC_CUDA_ALGO_SIMT;
@@ -385,6 +389,23 @@ int plan_scratch(NumcCtx *ctx, NumcDType dt, Plan *plan, size_t M, size_t K, siz
     }
   }
   return ctx_scratch(ctx, base + *ws_bytes + 256, s, out);
+}
+
+// After a wait for the context's stream: whether an integer digit GEMM of this
+// call or of an earlier, asynchronous one of the context abandoned a bounded wait.
+// The device's status word would do neither: its read waits for the stream (15 us
+// after a call's own wait: int16 100 x 1000 x 100 from host arrays 57 us, 41 with
+// this), and it holds other streams' failures.
+int ctx_failure(NumcCtx *ctx, const char *what) {
+  const unsigned st = numc_k::failure_word_take(ctx->failure);
+  if (st) return NUMC_SET_ERROR(NUMC_ERR_INTERNAL, "%s kernel abandoned a bounded wait (code %u)", what, st);
+  return 0;
+}
+
+// The dtypes of the integer digit GEMM.
+bool wide_integer(NumcDType dt) {
+  return dt != NUMC_DTYPE_INT8 && dt != NUMC_DTYPE_UINT8 && dt != NUMC_DTYPE_FLOAT32 &&
+         dt != NUMC_DTYPE_FLOAT64;
 }
 
 bool is_resident(const NumcArray *a) {
@@ -668,7 +689,7 @@ int matmul_impl(const NumcArray *a, const NumcArray *b, NumcArray *out, int algo
   // The fused epilogues add the bias themselves; the others get one pass.
   numc_k::Gemm gk = g;
   if (plan.algo != kAlgoIntDigits && !numc_k::fuses_bias(plan.algo)) gk.bias = nullptr;
-  if ((err = run_plan(dt, plan, gk, scratch + off_w, ws_bytes, s))) return err;
+  if ((err = run_plan(dt, plan, gk, scratch + off_w, ws_bytes, s, ctx->failure))) return err;
   if (g.bias && !gk.bias) {
     cudaError_t be = numc_k::launch_bias_add(dt, g, s);
     if (be != cudaSuccess) return cuda_fail(be, "bias add");
@@ -683,9 +704,9 @@ int matmul_impl(const NumcArray *a, const NumcArray *b, NumcArray *out, int algo
     CU(xfer_async(out->data, dout, so, cudaMemcpyDeviceToHost, s), "copy out to host");
     CU(cudaStreamSynchronize(s), "cudaStreamSynchronize");
   }
+  if (wide_integer(dt)) return ra && rb && ro ? 0 : ctx_failure(ctx, "matmul");
   if (plan.algo == NUMC_CUDA_ALGO_SPLIT_BF16 || plan.algo == NUMC_CUDA_ALGO_SPLIT_FP16 ||
-      plan.algo == NUMC_CUDA_ALGO_OZAKI || plan.algo == NUMC_CUDA_ALGO_TC_INT8 ||
-      plan.algo == kAlgoIntDigits) {
+      plan.algo == NUMC_CUDA_ALGO_OZAKI || plan.algo == NUMC_CUDA_ALGO_TC_INT8) {
     unsigned st = 0;
     CU(numc_k::read_and_clear_status(&st, s), "status read");
     if (st) return NUMC_SET_ERROR(NUMC_ERR_INTERNAL, "matmul kernel abandoned a bounded wait (code %u)", st);
@@ -792,6 +813,8 @@ void ctx_release_device(NumcCtx *ctx, const ArenaPos *keep_upto) {
     }
     ctx->scratch = nullptr;
     ctx->scratch_bytes = 0;
+    numc_k::failure_word_free(ctx->failure);
+    ctx->failure = nullptr;
     if (ctx->stream) cudaStreamDestroy((cudaStream_t)ctx->stream);
     ctx->stream = nullptr;
     for (void **cs : {&ctx->copy_in, &ctx->copy_out, &ctx->gemm2, &ctx->gemm3}) {
@@ -961,7 +984,7 @@ int bmm_impl(const NumcArray *a, const NumcArray *b, NumcArray *out) {
     g.rsa = a->strides[d - 2] / es; g.csa = a->strides[d - 1] / es;
     g.rsb = b->strides[d - 2] / es; g.csb = b->strides[d - 1] / es;
     g.rso = out->strides[d - 2] / es; g.cso = out->strides[d - 1] / es;
-    if ((err = run_plan(dt, plan, g, scratch + off_w, ws_bytes, s))) return err;
+    if ((err = run_plan(dt, plan, g, scratch + off_w, ws_bytes, s, ctx->failure))) return err;
   }
   if (ro) {
     out->residency = kDeviceOnly;
@@ -970,6 +993,7 @@ int bmm_impl(const NumcArray *a, const NumcArray *b, NumcArray *out) {
     CU(xfer_async(out->data, dout, so, cudaMemcpyDeviceToHost, s), "copy out to host");
     CU(cudaStreamSynchronize(s), "cudaStreamSynchronize");
   }
+  if (wide_integer(dt)) return ra && rb && ro ? 0 : ctx_failure(ctx, "bmm");
   if (plan.algo != NUMC_CUDA_ALGO_SIMT && plan.algo != NUMC_CUDA_ALGO_DMMA) {
     unsigned st = 0;
     CU(numc_k::read_and_clear_status(&st, s), "status read");
@@ -1132,7 +1156,7 @@ int dot_impl(const NumcArray *a, const NumcArray *b, NumcArray *out) {
                       : (dt == NUMC_DTYPE_FLOAT32 || dt == NUMC_DTYPE_FLOAT64) ? numc_k::kFloatNaive
                                                                                 : 0;
     if (gemm_branch) {
-      if ((err = run_plan(dt, plan, g, ws, ws_bytes, s))) return err;
+      if ((err = run_plan(dt, plan, g, ws, ws_bytes, s, ctx->failure))) return err;
     } else if (P == 1) {
       e = numc_k::launch_simt(dt, g, naive, s);
     } else {
@@ -1153,6 +1177,7 @@ int dot_impl(const NumcArray *a, const NumcArray *b, NumcArray *out) {
     CU(xfer_async(out->data, dout, so, cudaMemcpyDeviceToHost, s), "copy out to host");
     CU(cudaStreamSynchronize(s), "cudaStreamSynchronize");
   }
+  if (wide_integer(dt)) return ra && rb && ro ? 0 : ctx_failure(ctx, "dot");
   if (gemm_branch && plan.algo != NUMC_CUDA_ALGO_SIMT && plan.algo != NUMC_CUDA_ALGO_DMMA) {
     unsigned st = 0;
     CU(numc_k::read_and_clear_status(&st, s), "status read");
@@ -1324,6 +1349,7 @@ extern "C" int numc_cuda_array_to_host(NumcArray *arr) {
   size_t span = array_span_bytes(arr);
   if (span) CU(xfer_async(arr->data, arr->dev_base, span, cudaMemcpyDeviceToHost, s), "copy to host");
   CU(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+  if ((err = ctx_failure(arr->ctx, "an integer product's"))) return err;
   arr->residency = kBoth;
   return 0;
 }
@@ -1445,7 +1471,7 @@ extern "C" int numc_cuda_ctx_synchronize(NumcCtx *ctx) {
   if (!ctx) return NUMC_SET_ERROR(NUMC_ERR_NULL, "synchronize: ctx is NULL");
   if (!ctx->stream) return 0;
   CU(cudaStreamSynchronize((cudaStream_t)ctx->stream), "cudaStreamSynchronize");
-  return 0;
+  return ctx_failure(ctx, "an integer product's");
 }
 
 extern "C" size_t numc_cuda_gemm_workspace_size(NumcDType dt, int algo, int param,
@@ -1507,6 +1533,8 @@ extern "C" int numc_cuda_check_status(void *stream) {
   // own report through the library's static word.
   CU((cudaError_t)numc_k::static_status_read_and_clear(&st_static, stream), "status read");
   if (!st) st = st_static;
+  const unsigned st_ctx = numc_k::failure_words_take_all();   // contexts' integer products
+  if (!st) st = st_ctx;
   if (st) return NUMC_SET_ERROR(NUMC_ERR_INTERNAL, "a kernel abandoned a bounded wait (code %u)", st);
   return 0;
 }

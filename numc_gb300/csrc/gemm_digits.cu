@@ -1080,11 +1080,10 @@ double int_digits_gain_us(NumcDType dt, int64_t M, int64_t K, int64_t N) {
 }
 
 cudaError_t launch_int_digits(NumcDType dt, const Gemm &g, void *ws, size_t ws_bytes,
-                              cudaStream_t s) {
+                              unsigned *status, cudaStream_t s) {
   const int bytes = int_bytes(dt);
   const IntPlan p = int_plan(bytes, g.M, g.K, g.N);
   if (!bytes || !p.BN || ws_bytes < p.total || ((uintptr_t)ws & 255)) return cudaErrorInvalidValue;
-  unsigned *status = status_word();
   if (!status) return cudaErrorMemoryAllocation;
   if (bytes == 8) return run_int<unsigned long long>(g, p, (char *)ws, status, s);
   if (bytes == 4) return run_int<unsigned>(g, p, (char *)ws, status, s);

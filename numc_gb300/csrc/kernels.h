@@ -151,12 +151,13 @@ cudaError_t launch_ozaki(const Gemm &g, int slices, void *ws, size_t ws_bytes,
 
 // 16-, 32- and 64-bit integers as digit products on tcgen05, modulo 2^bits.
 // Workspace bytes, or 0 where the CUDA-core kernel is the faster one (or the
-// only one); the launcher takes the problems with a workspace.
+// only one); the launcher takes the problems with a workspace.  `status`: the word
+// that a kernel which abandons a bounded wait writes.
 size_t int_digits_workspace(NumcDType dt, int64_t M, int64_t K, int64_t N);
 // Estimated time it saves over the CUDA cores, in us.
 double int_digits_gain_us(NumcDType dt, int64_t M, int64_t K, int64_t N);
 cudaError_t launch_int_digits(NumcDType dt, const Gemm &g, void *ws, size_t ws_bytes,
-                              cudaStream_t s);
+                              unsigned *status, cudaStream_t s);
 
 // numc_array_rand's generator (rand.cu): numc's four-lane xoshiro256**
 // state of the calling host thread, and numc's OpenMP maximum thread count

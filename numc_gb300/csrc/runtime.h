@@ -76,6 +76,7 @@ struct NumcCtx {
   int device;                         // device the stream belongs to
   void *scratch;                      // device scratch (staging, splits)
   size_t scratch_bytes;
+  unsigned *failure;                  // integer digit GEMMs' failure word (pinned, lazy)
   std::vector<numc_rt::DeviceAlloc> *dev_allocs;
   std::vector<numc_rt::DeviceSlab> *dev_slabs;
   size_t dev_cur;                     // slab that bump allocation continues in

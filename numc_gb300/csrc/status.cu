@@ -4,8 +4,10 @@
 // nonzero code in a per-device status word and return, so that a broken
 // pipeline surfaces as NUMC_ERR_INTERNAL instead of a hung GPU.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <vector>
 
 #include "kernels.h"
 #include "status.h"
@@ -19,6 +21,8 @@ std::atomic<int> g_wait_starve{0};
 std::atomic<int> g_fail_mallocs{0};
 std::mutex g_status_mu;
 unsigned *g_status_dev[64] = {nullptr};
+std::mutex g_failure_mu;
+std::vector<unsigned *> g_failure_words;
 }  // namespace
 
 void count_launch(unsigned n) { g_launches.fetch_add(n); }
@@ -63,6 +67,40 @@ cudaError_t read_and_clear_status(unsigned *status, cudaStream_t s) {
   if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, sizeof(unsigned), s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return e;
+}
+
+unsigned *failure_word_alloc() {
+  unsigned *p = nullptr;
+  if (cudaHostAlloc((void **)&p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  *p = 0;
+  std::lock_guard<std::mutex> lock(g_failure_mu);
+  g_failure_words.push_back(p);
+  return p;
+}
+
+void failure_word_free(unsigned *word) {
+  if (!word) return;
+  std::lock_guard<std::mutex> lock(g_failure_mu);
+  g_failure_words.erase(std::find(g_failure_words.begin(), g_failure_words.end(), word));
+  cudaFreeHost(word);
+}
+
+unsigned failure_word_take(unsigned *word) {
+  return word ? __atomic_exchange_n(word, 0u, __ATOMIC_ACQ_REL) : 0;
+}
+
+unsigned failure_words_take_all() {
+  std::lock_guard<std::mutex> lock(g_failure_mu);
+  unsigned first = 0;
+  for (unsigned *w : g_failure_words) {
+    const unsigned st = failure_word_take(w);
+    if (!first) first = st;
+  }
+  return first;
 }
 
 }  // namespace numc_k

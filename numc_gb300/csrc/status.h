@@ -9,6 +9,16 @@ namespace numc_k {
 // use), or nullptr if it could not be allocated.
 unsigned *status_word();
 
+// A context's own failure word, for kernels whose calls do not wait for them:
+// pinned host memory that the kernels write and the host reads, without a copy, at
+// the context's next wait.  nullptr if it could not be allocated.
+unsigned *failure_word_alloc();
+void failure_word_free(unsigned *word);
+// Its code, cleared (0: no failure).
+unsigned failure_word_take(unsigned *word);
+// The first code of any context's word, all of them cleared.
+unsigned failure_words_take_all();
+
 // Codes written to the status word (first writer wins).
 enum StatusCode : unsigned {
   kStatusOk = 0,

@@ -1,0 +1,130 @@
+"""16- to 64-bit integer products of a context's arrays, which take the tensor
+cores where those are faster: resident calls only enqueue work, a batch takes
+them as one product does, and failures and refused memory stay with the context
+that met them."""
+import numpy as np
+import pytest
+
+import numc_gb300 as nc
+import oracle
+
+from gpu_util import needs_gpu
+
+pytestmark = [pytest.mark.gpu, needs_gpu]
+torch = pytest.importorskip("torch")
+
+DTYPES = ["int16", "int32", "int64"]
+LIMIT_NS = 20_000_000   # 20 ms per abandoned wait
+
+
+def _rand(dt, shape, seed):
+    info = np.iinfo(dt)
+    return np.random.default_rng(seed).integers(info.min, info.max, shape, dtype=dt, endpoint=True)
+
+
+class starved_waits:
+    """Bounded waits run out after LIMIT_NS: the producers issue no loads."""
+
+    def __enter__(self):
+        torch.cuda.synchronize()
+        nc.lib().numc_cuda_debug_wait_timeout(LIMIT_NS, 1)
+
+    def __exit__(self, *exc):
+        torch.cuda.synchronize()
+        nc.lib().numc_cuda_debug_wait_timeout(0, 0)
+
+
+def _internal(call):
+    with pytest.raises(nc.NumcError) as ei:
+        call()
+    assert ei.value.code == nc.ERR_INTERNAL
+    assert "bounded wait" in ei.value.msg
+
+
+def _call(op, ctx, dt, n, resident):
+    """(call, output array, expected result) of an n^3 product or two of them."""
+    if op == "bmm":
+        x, w = _rand(dt, (2, n, n), 1), _rand(dt, (2, n, n), 2)
+        want = np.stack([oracle.matmul(x[i], w[i]) for i in range(2)])
+    else:
+        x, w = _rand(dt, (n, n), 1), _rand(dt, (n, n), 2)
+        want = oracle.matmul(x, w)
+    X, W, O = ctx.from_numpy(x), ctx.from_numpy(w), ctx.zeros(want.shape, dt)
+    bias = ctx.from_numpy(np.ones(n, dt)) if op == "linear" else None
+    if bias is not None:
+        with np.errstate(over="ignore"):
+            want = want + np.ones(n, dt)
+    if resident:
+        for t in (X, W, O) + ((bias,) if bias else ()):
+            t.to_device()
+    fn = {"matmul": nc.matmul, "dot": nc.dot, "bmm": nc.bmm}.get(op)
+    return (lambda: fn(X, W, O) if fn else nc.linear(X, W, bias, O)), O, want
+
+
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("op", ["matmul", "linear", "bmm", "dot"])
+def test_resident_calls_only_enqueue(op, dt):
+    with nc.Ctx() as ctx:
+        call, out, want = _call(op, ctx, dt, 1024, True)
+        call()                  # scratch grows to its size here
+        ctx.synchronize()
+        s = torch.cuda.ExternalStream(ctx.stream())
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(400_000_000)   # about 0.2 s
+        n = nc.launch_count()
+        call()
+        assert not s.query(), "the call waited for its stream"
+        assert nc.launch_count() - n == (4 if op == "bmm" else 2)   # the tensor cores' two
+        out.to_host()
+        np.testing.assert_array_equal(out.numpy(), want)
+
+
+@pytest.mark.parametrize("resident", [False, True])
+def test_failures_of_other_streams_stay_there(resident):
+    """An integer product neither reports nor clears what another stream's kernel
+    recorded."""
+    a = torch.rand((300, 520), device="cuda")
+    b = torch.rand((520, 270), device="cuda")
+    c = torch.zeros((300, 270), device="cuda")
+    with nc.Ctx() as ctx:
+        call, out, want = _call("matmul", ctx, "int32", 1024, resident)
+        with starved_waits():
+            nc.gemm(a, b, c, algo=nc.ALGO_SPLIT_FP16)
+        call()
+        out.to_host()
+        np.testing.assert_array_equal(out.numpy(), want)
+        _internal(nc.check_status)
+        nc.check_status()
+
+
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("op", ["matmul", "linear", "bmm", "dot"])
+def test_host_call_reports_its_own_failure(op, dt):
+    with nc.Ctx() as ctx, nc.Ctx() as other:
+        call, out, want = _call(op, ctx, dt, 640, False)
+        call2, out2, want2 = _call("matmul", other, dt, 640, False)
+        with starved_waits():
+            _internal(call)
+        call2()
+        np.testing.assert_array_equal(out2.numpy(), want2)
+        call()
+        np.testing.assert_array_equal(out.numpy(), want)
+        nc.check_status()
+
+
+@pytest.mark.parametrize("where", ["to_host", "synchronize", "check_status", "host_call"])
+def test_resident_call_reports_at_the_next_wait(where):
+    with nc.Ctx() as ctx:
+        call, out, want = _call("matmul", ctx, "int32", 1024, True)
+        small = ctx.from_numpy(np.eye(1024, 4, dtype="int32"))   # a CUDA-core product
+        res = ctx.zeros((1024, 4), "int32")
+        with starved_waits():
+            call()
+        wait = {"to_host": out.to_host, "synchronize": ctx.synchronize,
+                "check_status": nc.check_status, "host_call": lambda: nc.matmul(out, small, res)}
+        _internal(wait[where])
+        call()
+        wait[where]()
+        out.to_host()
+        np.testing.assert_array_equal(out.numpy(), want)
+        nc.check_status()
