@@ -369,19 +369,18 @@ int ctx_scratch(NumcCtx *ctx, size_t bytes, cudaStream_t s, char **out) {
 
 // Scratch of `base` bytes for staged operands plus the plan's workspace
 // (*ws_bytes).  Integer plans give the tensor cores up for the CUDA cores,
-// which need no workspace, where the device has no room for the digits, where
+// which need no workspace, where the device has no room for the digits and where
 // the stream is being captured (the digits would lie in scratch that a later call
-// may free), and, with an asynchronous result (`async`: a resident output and
-// inputs), where they would not save 15 us.
+// may free).
 int plan_scratch(NumcCtx *ctx, NumcDType dt, Plan *plan, size_t M, size_t K, size_t N,
-                 size_t base, bool async, cudaStream_t s, size_t *ws_bytes, char **out) {
+                 size_t base, cudaStream_t s, size_t *ws_bytes, char **out) {
   *ws_bytes = plan_workspace(dt, *plan, M, K, N);
   if (plan->algo == kAlgoIntDigits) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     const bool captured =
         cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
     if (!ctx->failure && !captured) ctx->failure = numc_k::failure_word_alloc();
-    if (captured || !ctx->failure || (async && numc_k::int_digits_gain_us(dt, M, K, N) < 15) ||
+    if (captured || !ctx->failure ||
         grow_scratch(ctx, base + *ws_bytes + 256, s) != cudaSuccess) {
       cudaGetLastError();
       plan->algo = NUMC_CUDA_ALGO_SIMT;
@@ -661,8 +660,7 @@ int matmul_impl(const NumcArray *a, const NumcArray *b, NumcArray *out, int algo
   size_t off_w = off_bias + align_up(rbias ? 0 : sbias, 256);
   size_t ws_bytes = 0;
   char *scratch = nullptr;
-  if ((err = plan_scratch(ctx, dt, &plan, M, K, N, off_w, ra && rb && ro, s, &ws_bytes,
-                          &scratch))) return err;
+  if ((err = plan_scratch(ctx, dt, &plan, M, K, N, off_w, s, &ws_bytes, &scratch))) return err;
 
   const char *da = ra ? a->dev_base : scratch + off_a;
   const char *db = rb ? b->dev_base : scratch + off_b;
@@ -960,8 +958,7 @@ int bmm_impl(const NumcArray *a, const NumcArray *b, NumcArray *out) {
   const size_t off_w = off_o + align_up(ro ? 0 : so, 256);
   size_t ws_bytes = 0;
   char *scratch = nullptr;
-  if ((err = plan_scratch(ctx, dt, &plan, M, K, N, off_w, ra && rb && ro, s, &ws_bytes,
-                          &scratch))) return err;
+  if ((err = plan_scratch(ctx, dt, &plan, M, K, N, off_w, s, &ws_bytes, &scratch))) return err;
   const char *da = ra ? a->dev_base : scratch;
   const char *db = rb ? b->dev_base : scratch + off_b;
   char *dout = ro ? out->dev_base : scratch + off_o;
@@ -1113,8 +1110,7 @@ int dot_impl(const NumcArray *a, const NumcArray *b, NumcArray *out) {
   const size_t off_o = off_b + align_up(rb ? 0 : sb, 256);
   const size_t off_w = off_o + align_up(ro ? 0 : so, 256);
   char *scratch = nullptr;
-  if (gemm_branch) err = plan_scratch(ctx, dt, &plan, M, K, N, off_w, ra && rb && ro, s, &ws_bytes,
-                          &scratch);
+  if (gemm_branch) err = plan_scratch(ctx, dt, &plan, M, K, N, off_w, s, &ws_bytes, &scratch);
   else err = ctx_scratch(ctx, off_w + ws_bytes + 256, s, &scratch);
   if (err) return err;
   const char *da = ra ? a->dev_base : scratch;

@@ -1074,11 +1074,6 @@ size_t int_digits_workspace(NumcDType dt, int64_t M, int64_t K, int64_t N) {
   return p.BN && p.us < p.simt_us ? p.total : 0;
 }
 
-double int_digits_gain_us(NumcDType dt, int64_t M, int64_t K, int64_t N) {
-  const IntPlan p = int_plan(int_bytes(dt), M, K, N);
-  return p.BN ? p.simt_us - p.us : 0;
-}
-
 cudaError_t launch_int_digits(NumcDType dt, const Gemm &g, void *ws, size_t ws_bytes,
                               unsigned *status, cudaStream_t s) {
   const int bytes = int_bytes(dt);

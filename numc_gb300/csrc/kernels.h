@@ -154,8 +154,6 @@ cudaError_t launch_ozaki(const Gemm &g, int slices, void *ws, size_t ws_bytes,
 // only one); the launcher takes the problems with a workspace.  `status`: the word
 // that a kernel which abandons a bounded wait writes.
 size_t int_digits_workspace(NumcDType dt, int64_t M, int64_t K, int64_t N);
-// Estimated time it saves over the CUDA cores, in us.
-double int_digits_gain_us(NumcDType dt, int64_t M, int64_t K, int64_t N);
 cudaError_t launch_int_digits(NumcDType dt, const Gemm &g, void *ws, size_t ws_bytes,
                               unsigned *status, cudaStream_t s);
 

@@ -128,3 +128,18 @@ def test_resident_call_reports_at_the_next_wait(where):
         out.to_host()
         np.testing.assert_array_equal(out.numpy(), want)
         nc.check_status()
+
+
+def test_resident_batch_takes_the_tensor_cores():
+    """8 products that gain a few us each."""
+    n, P = 512, 8
+    x, w = _rand("int32", (P, n, n), 3), _rand("int32", (P, n, n), 4)
+    with nc.Ctx() as ctx:
+        X, W, O = ctx.from_numpy(x), ctx.from_numpy(w), ctx.zeros((P, n, n), "int32")
+        for t in (X, W, O):
+            t.to_device()
+        k = nc.launch_count()
+        nc.bmm(X, W, O)
+        assert nc.launch_count() - k == 2 * P
+        O.to_host()
+        np.testing.assert_array_equal(O.numpy(), np.stack([oracle.matmul(x[i], w[i]) for i in range(P)]))
