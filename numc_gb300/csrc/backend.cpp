@@ -346,25 +346,47 @@ int ctx_stream(NumcCtx *ctx, cudaStream_t *s) {
   return 0;
 }
 
-cudaError_t grow_scratch(NumcCtx *ctx, size_t bytes, cudaStream_t s) {
-  if (ctx->scratch_bytes >= bytes) return cudaSuccess;
-  cudaError_t e;
-  if (ctx->scratch) {
-    if ((e = cudaStreamSynchronize(s))) return e;
-    cudaFree(ctx->scratch);
-    ctx->scratch = nullptr;
-    ctx->scratch_bytes = 0;
-  }
-  size_t grow = align_up(bytes + bytes / 4, 1 << 20);
-  if ((e = numc_k::dev_malloc(&ctx->scratch, grow))) return e;
-  ctx->scratch_bytes = grow;
-  return cudaSuccess;
-}
+size_t scratch_growth(size_t bytes) { return align_up(bytes + bytes / 4, 1 << 20); }
 
 int ctx_scratch(NumcCtx *ctx, size_t bytes, cudaStream_t s, char **out) {
-  CU(grow_scratch(ctx, bytes, s), "cudaMalloc(scratch)");
+  if (ctx->scratch_bytes < bytes) {
+    if (ctx->scratch) {
+      CU(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+      cudaFree(ctx->scratch);
+      ctx->scratch = nullptr;
+      ctx->scratch_bytes = 0;
+    }
+    const size_t grow = scratch_growth(bytes);
+    CU(numc_k::dev_malloc(&ctx->scratch, grow), "cudaMalloc(scratch)");
+    ctx->scratch_bytes = grow;
+  }
   *out = (char *)ctx->scratch;
   return 0;
+}
+
+// Grows the scratch for a call that can do without: the larger buffer comes first,
+// so that a refusal leaves the context what it has, and a size that was refused is
+// not asked for again until the context gives device memory back.
+bool try_grow_scratch(NumcCtx *ctx, size_t bytes, cudaStream_t s) {
+  if (ctx->scratch_bytes >= bytes) return true;
+  if (ctx->scratch_refused && bytes >= ctx->scratch_refused) return false;
+  const size_t grow = scratch_growth(bytes);
+  void *p = nullptr;
+  if (numc_k::dev_malloc(&p, grow) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->scratch_refused = bytes;
+    return false;
+  }
+  if (ctx->scratch) {
+    if (cudaStreamSynchronize(s) != cudaSuccess) {   // its users' failure; theirs to report
+      cudaFree(p);
+      return false;
+    }
+    cudaFree(ctx->scratch);
+  }
+  ctx->scratch = p;
+  ctx->scratch_bytes = grow;
+  return true;
 }
 
 // Scratch of `base` bytes for staged operands plus the plan's workspace
@@ -381,8 +403,7 @@ int plan_scratch(NumcCtx *ctx, NumcDType dt, Plan *plan, size_t M, size_t K, siz
         cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
     if (!ctx->failure && !captured) ctx->failure = numc_k::failure_word_alloc();
     if (captured || !ctx->failure ||
-        grow_scratch(ctx, base + *ws_bytes + 256, s) != cudaSuccess) {
-      cudaGetLastError();
+        !try_grow_scratch(ctx, base + *ws_bytes + 256, s)) {
       plan->algo = NUMC_CUDA_ALGO_SIMT;
       *ws_bytes = 0;
     }
@@ -781,6 +802,7 @@ int device_copy_contiguous(const NumcArray *src, NumcArray *dst) {
 
 void ctx_release_device(NumcCtx *ctx, const ArenaPos *keep_upto) {
   if (!ctx->dev_allocs) return;
+  ctx->scratch_refused = 0;
   if (ctx->stream && !ctx->dev_allocs->empty())
     cudaStreamSynchronize((cudaStream_t)ctx->stream);
   auto &v = *ctx->dev_allocs;

@@ -137,6 +137,7 @@ extern "C" NumcCtx *numc_ctx_create(void) {
   ctx->device = -1;
   ctx->scratch = nullptr;
   ctx->scratch_bytes = 0;
+  ctx->scratch_refused = 0;
   ctx->failure = nullptr;
   ctx->dev_allocs = new (std::nothrow) std::vector<DeviceAlloc>();
   ctx->dev_slabs = new (std::nothrow) std::vector<DeviceSlab>();

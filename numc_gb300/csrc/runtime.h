@@ -76,6 +76,7 @@ struct NumcCtx {
   int device;                         // device the stream belongs to
   void *scratch;                      // device scratch (staging, splits)
   size_t scratch_bytes;
+  size_t scratch_refused;             // smallest optional size the device refused (0: none)
   unsigned *failure;                  // integer digit GEMMs' failure word (pinned, lazy)
   std::vector<numc_rt::DeviceAlloc> *dev_allocs;
   std::vector<numc_rt::DeviceSlab> *dev_slabs;

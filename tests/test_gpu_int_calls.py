@@ -143,3 +143,30 @@ def test_resident_batch_takes_the_tensor_cores():
         assert nc.launch_count() - k == 2 * P
         O.to_host()
         np.testing.assert_array_equal(O.numpy(), np.stack([oracle.matmul(x[i], w[i]) for i in range(P)]))
+
+
+def test_no_room_for_the_digits():
+    """The device refuses the digits' memory: the context keeps the scratch that it
+    has, the CUDA cores take the call, and the next one does not ask again."""
+    n = 640
+    a, b = _rand("int32", (n, n), 5), _rand("int32", (n, n), 6)
+    want = oracle.matmul(a, b)
+    with nc.Ctx() as ctx:
+        A, B, C = ctx.from_numpy(a), ctx.from_numpy(b), ctx.zeros((n, n), "int32")
+        nc.matmul_naive(A, B, C)          # scratch for the staged operands alone
+        nc.lib().numc_cuda_debug_fail_malloc(1000)
+        try:
+            for _ in range(2):
+                C.write(np.zeros_like(want))
+                k = nc.launch_count()
+                nc.matmul(A, B, C)
+                assert nc.launch_count() - k == 1
+                np.testing.assert_array_equal(C.numpy(), want)
+            # one allocation would fail, and the call makes none
+            nc.lib().numc_cuda_debug_fail_malloc(1)
+            nc.matmul(A, B, C)
+            with pytest.raises(nc.NumcError) as ei:
+                A.to_device()
+            assert ei.value.code == nc.ERR_MALLOC
+        finally:
+            nc.lib().numc_cuda_debug_fail_malloc(0)
