@@ -65,6 +65,10 @@ __device__ __forceinline__ void copy4(uint32_t dst, const float *src, int bytes 
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes));
 }
 
+__device__ __forceinline__ void store4(uint32_t dst, float x) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst), "f"(x));
+}
+
 // The copies of one tile's slabs by a block's threads.  The last tiles move inside
 // the matrix, so that no load needs a check of rows or columns: they compute some
 // outputs of their neighbours again and leave them unstored.  A matrix narrower
@@ -128,6 +132,14 @@ struct F32Loads {
     }
     pa += step_a;
     pb += step_b;
+  }
+  // -0 for the zeros that this thread's own copies, complete, wrote past K in B's part
+  // of the stage at `sa`: fma(+0, -0, x) is x, -0 included.
+  __device__ __forceinline__ void past_k(uint32_t sa, int left) const {
+    const uint32_t sb = sa + BK * Cfg::APITCH * 4;
+#pragma unroll
+    for (int q = 0; q < LB; q++)
+      if (b_kk(q) >= left) store4(sb + (b_kk(q) * Cfg::BPITCH + b_col(q)) * 4, -0.0f);
   }
 };
 
@@ -220,10 +232,11 @@ struct F32Acc {
     }
   }
 
-  // The end of slab t of `slabs`: remainder outputs at the end of their K block.
+  // The end of slab t of `slabs`: remainder outputs at the end of a K block but the
+  // last, which to_shared adds.
   // bsum: the tile's edge sums, THREADS apart, this thread's first.
   __device__ __forceinline__ void end_slab(int64_t t, int64_t slabs, float *bsum) {
-    if (!(edge_i | edge_j) || ((t + 1) * BK % simt::kNumcKC != 0 && t + 1 != slabs)) return;
+    if (!(edge_i | edge_j) || (t + 1) * BK % simt::kNumcKC != 0 || t + 1 == slabs) return;
     const bool first = t < simt::kNumcKC / BK;
 #pragma unroll
     for (int i = 0; i < TM; i++)
@@ -247,7 +260,7 @@ struct F32Acc {
 #pragma unroll
         for (int j = 0; j < TN; j++)
           if (is_edge(i, j)) {
-            const u64 v = __float_as_uint(bsum[(i * TN + j) * THREADS]);
+            const u64 v = __float_as_uint(simt::add_rn<float>(bsum[(i * TN + j) * THREADS], output(i, j)));
             acc[i][j / 2] = j & 1 ? (acc[i][j / 2] & 0xffffffffull) | v << 32
                                   : (acc[i][j / 2] & 0xffffffff00000000ull) | v;
           }
@@ -270,6 +283,14 @@ struct F32Acc {
 // the operand's strides and alignment allow it.  SMALL is numc's unpacked path
 // (its narrow tiles' scalar columns round product and sum separately); else the
 // packed path, remainder outputs summed per 256-deep K block in registers.
+//
+// Of a last slab only the steps below K may count: one past it, fma(0, 0, x), makes
+// +0 of a chain that ended in -0, as numc's does where every product underflows
+// from below.  Those steps run in a loop of their own (20 x 3 x 20 3.5 -> 2.8 us,
+// 150 x 127 x 150 3.6 -> 3.9, 500 grouped problems of 16 to 256 135 -> 118), except with
+// 4 x 4 outputs and 16-byte copies of both operands, where that loop spoils the
+// order of the main one (512^3 13.8 -> 14.9): there B's rows past K are kPastK, and
+// fma(+0, -0, x) is x.
 // Measured, us before (2 x 2 outputs of 32 x 32 tiles, element copies) and after:
 //   96^3 4.3 / 3.2, 128^3 4.5 / 3.0, 256 x 784 x 128 17.7 / 9.8, 64 x 1000 x 64 22 / 11.5,
 //   512^3 18.7 / 14.0, 200 x 3000 x 200 67 / 36.5, 700^3 51 / 29.
@@ -288,6 +309,8 @@ __device__ __forceinline__ void copy16(uint32_t dst, const float *src, int bytes
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes));
 }
 
+static __device__ const float4 kPastK = {-0.0f, -0.0f, -0.0f, -0.0f};
+
 template <int TY, int TX, int TM, int TN, bool SMALL, bool VA, bool VB>
 __device__ __forceinline__ void f32_small_tile(const Gemm &g, int64_t m0, int64_t n0, float *smem) {
   using Cfg = F32SmallCfg<TY, TX, TM, TN>;
@@ -297,8 +320,9 @@ __device__ __forceinline__ void f32_small_tile(const Gemm &g, int64_t m0, int64_
   const int mr = (int)min((int64_t)BM, g.M - m0) - 1, nr = (int)min((int64_t)BN, g.N - n0) - 1;
   const bool a_k = g.csa == 1, b_n = g.csb == 1 || g.rsb != 1;
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+  constexpr bool PAD = TM == 4 && VA && VB;   // kPastK past K, no loop for a part of a slab
   // Rows and columns past the matrix repeat the last one (in 16-byte copies:
-  // columns past it are zeros); k past K is zeros, from an address inside.
+  // columns past it are zeros); k past K is zeros (but PAD), from an address inside.
   // Strides fit 32 bits (the launcher checks).
   const float *pa = A + m0 * g.rsa, *pb = B + n0 * g.csb;
   const int rsa = (int)g.rsa, csa = (int)g.csa, rsb = (int)g.rsb, csb = (int)g.csb;
@@ -325,7 +349,9 @@ __device__ __forceinline__ void f32_small_tile(const Gemm &g, int64_t m0, int64_
       for (int q = 0; q < BK * BN / 4 / THREADS; q++) {
         const int e = tid + q * THREADS, k = e / (BN / 4), c = e % (BN / 4) * 4;
         const int n = full || k < left ? max(0, min(4, nr + 1 - c)) : 0;
-        copy16(sb + (k * Cfg::BPITCH + c) * 4, n ? pb + k * rsb + c : pb, 4 * n);
+        const bool past = PAD && !full && k >= left;
+        copy16(sb + (k * Cfg::BPITCH + c) * 4, past ? &kPastK.x : n ? pb + k * rsb + c : pb,
+               past ? 16 : 4 * n);
       }
     } else {
 #pragma unroll
@@ -360,22 +386,38 @@ __device__ __forceinline__ void f32_small_tile(const Gemm &g, int64_t m0, int64_
         if (m0 + row_of(i) >= er || n0 + col_of(j) >= ec) edge |= 1u << (i * TN + j);
   }
 
+  auto step = [&](float a, float b, float x, int j) {
+    return SMALL && (unfused >> j & 1) ? simt::madd_unfused(a, b, x) : __fmaf_rn(a, b, x);
+  };
+  auto end_block = [&](int t) {   // remainder outputs at the end of their K block, in slab t
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < TN; j++)
+        if (edge >> (i * TN + j) & 1) {
+          bsum[i][j] = t < simt::kNumcKC / BK ? acc[i][j] : simt::add_rn<float>(bsum[i][j], acc[i][j]);
+          acc[i][j] = 0.0f;
+        }
+  };
   const int slabs = (int)((g.K + BK - 1) / BK);
 #pragma unroll
   for (int t = 0; t < Cfg::STAGES - 1; t++) {
     if (t < slabs) load(t, (int)g.K - t * BK);
     asm volatile("cp.async.commit_group;");
   }
-  for (int t = 0; t < slabs; t++) {
+  const int whole = PAD ? slabs : (int)g.K / BK;
+  for (int t = 0; t < whole; t++) {
     asm volatile("cp.async.wait_group %0;" ::"n"(Cfg::STAGES - 2) : "memory");
     __syncthreads();   // slab t has arrived, and everyone is done with slab t - 1
     const int tn = t + Cfg::STAGES - 1;
     if (tn < slabs) load(tn % Cfg::STAGES, (int)g.K - tn * BK);
     asm volatile("cp.async.commit_group;");
     const float *As = smem + t % Cfg::STAGES * Cfg::STAGE, *Bs = As + BM * Cfg::APITCH;
-    // 4 x 4 outputs: operands of the next four k are read while this four's
-    // FMAs run (2 x 2: the compiler's own order is the faster one)
-    constexpr int P = TM * TN > 4 ? 2 : 1;
+    // Operands of the next four k are read while this four's FMAs run (2 x 2 outputs
+    // and element copies: the compiler's own order is the faster one, 12.2
+    // against 16.0 us for 255 x 783 x 127; 2 x 2 and 16-byte copies: 9.6 against 13.1
+    // for 256 x 784 x 128).
+    constexpr int P = TM * TN > 4 || (VA && VB) ? 2 : 1;
     float av[P][TM][4], bv[P][4][TN];
     auto fetch = [&](int k4) {
       float(&a)[TM][4] = av[k4 / 4 % P];
@@ -392,7 +434,10 @@ __device__ __forceinline__ void f32_small_tile(const Gemm &g, int64_t m0, int64_
       }
     };
     if (P == 2) fetch(0);
-#pragma unroll
+    // (the unpacked path's problems are a few slabs: fetching the code of a whole
+    // one's steps took longer than running it, 96^3 5.2 -> 4.2 us, the same 500
+    // grouped problems 118 -> 107)
+#pragma unroll (SMALL ? 4 : BK / 4)
     for (int k4 = 0; k4 < BK; k4 += 4) {
       if (P == 1) fetch(k4);
       else if (k4 + 4 < BK) fetch(k4 + 4);
@@ -403,23 +448,52 @@ __device__ __forceinline__ void f32_small_tile(const Gemm &g, int64_t m0, int64_
 #pragma unroll
         for (int i = 0; i < TM; i++)
 #pragma unroll
-          for (int j = 0; j < TN; j++) {
-            if constexpr (SMALL)
-              acc[i][j] = unfused >> j & 1 ? simt::madd_unfused(a[i][k], b[k][j], acc[i][j])
-                                           : __fmaf_rn(a[i][k], b[k][j], acc[i][j]);
-            else acc[i][j] = __fmaf_rn(a[i][k], b[k][j], acc[i][j]);
-          }
+          for (int j = 0; j < TN; j++) acc[i][j] = step(a[i][k], b[k][j], acc[i][j], j);
     }
-    if (!SMALL && edge && ((t + 1) * BK % simt::kNumcKC == 0 || t + 1 == slabs)) {
+    if (!SMALL && edge && ((t + 1) * BK % simt::kNumcKC == 0 || t + 1 == slabs)) end_block(t);
+  }
+  if (whole < slabs) {
+    // the last slab's steps below K, four at a time (unrolled: 25 x 829 x 274 14.2 ->
+    // 14.0 us; the unpacked path: see above)
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const float *a0 = smem + whole % Cfg::STAGES * Cfg::STAGE + row_of(0) * Cfg::APITCH;
+    const float *b0 = smem + whole % Cfg::STAGES * Cfg::STAGE + BM * Cfg::APITCH + col_of(0);
+    const int n = (int)g.K - whole * BK;
+    int k = 0;
+#pragma unroll (SMALL ? 1 : 4)
+    for (; k + 4 <= n; k += 4) {
+      float a[TM][4], b[4][TN];
+#pragma unroll
+      for (int i = 0; i < TM; i++)
+        *reinterpret_cast<float4 *>(a[i]) =
+            *reinterpret_cast<const float4 *>(a0 + i * TY * Cfg::APITCH + k);
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int j = 0; j < TN; j += 2)
+          *reinterpret_cast<float2 *>(b[q] + j) =
+              *reinterpret_cast<const float2 *>(b0 + (k + q) * Cfg::BPITCH + j);
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int i = 0; i < TM; i++)
+#pragma unroll
+          for (int j = 0; j < TN; j++) acc[i][j] = step(a[i][q], b[q][j], acc[i][j], j);
+    }
+#pragma unroll 1
+    for (; k < n; k++) {
+      float a[TM], b[TN];
+#pragma unroll
+      for (int i = 0; i < TM; i++) a[i] = a0[i * TY * Cfg::APITCH + k];
+#pragma unroll
+      for (int j = 0; j < TN; j++) b[j] = b0[k * Cfg::BPITCH + j];
 #pragma unroll
       for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int j = 0; j < TN; j++)
-          if (edge >> (i * TN + j) & 1) {
-            bsum[i][j] = t < simt::kNumcKC / BK ? acc[i][j] : simt::add_rn<float>(bsum[i][j], acc[i][j]);
-            acc[i][j] = 0.0f;
-          }
+        for (int j = 0; j < TN; j++) acc[i][j] = step(a[i], b[j], acc[i][j], j);
     }
+    if (!SMALL && edge) end_block(whole);
   }
 #pragma unroll
   for (int i = 0; i < TM; i++) {

@@ -47,8 +47,15 @@ __global__ void __launch_bounds__(TY * TX, CTAS) f32_gemm(const Gemm g, unsigned
     asm volatile("cp.async.commit_group;");
   }
   int stage = 0;
-  for (int64_t t = 0; t < slabs; t++) {
+  // Of a last slab only the steps below K may count (see F32SmallCfg): they run in a
+  // loop of their own (2000 x 17 x 2000 13.2 -> 12.0 us), whose code has to be fetched
+  // for it (2000 x 1999 x 1501, operands not in L2, 246.0 -> 248.9).  The 128 x 80 tile's deep
+  // products take B's steps past K as -0 instead (245.5; the other tiles' main
+  // loops get slower for it: 1000 x 999 x 1000 60.6 -> 64.0).
+  const int64_t whole = g.K / BK, last = TN == 10 && whole >= 16 ? slabs : whole;
+  for (int64_t t = 0; t < last; t++) {
     asm volatile("cp.async.wait_group %0;" ::"n"(Cfg::STAGES - 2) : "memory");
+    if (TN == 10 && t == whole) ld.past_k(sbase + stage * Cfg::STAGE * 4, (int)(g.K % BK));
     __syncthreads();   // slab t has arrived, and everyone is done with slab t - 1
     const int64_t tn = t + Cfg::STAGES - 1;
     const int into = stage == 0 ? Cfg::STAGES - 1 : stage - 1;
@@ -57,6 +64,11 @@ __global__ void __launch_bounds__(TY * TX, CTAS) f32_gemm(const Gemm g, unsigned
     acc.slab(smem + stage * Cfg::STAGE);
     if (++stage == Cfg::STAGES) stage = 0;
     acc.end_slab(t, slabs, bsum);
+  }
+  if (last < slabs) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    acc.part_slab(smem + stage * Cfg::STAGE, (int)(g.K % BK));
   }
   acc.to_shared(smem, bsum);
   store_tile<BM, BN, TY * TX>(g, smem, m0, n0, (int)(mt - m0), (int)(nt - n0));
