@@ -170,3 +170,50 @@ def test_no_room_for_the_digits():
             assert ei.value.code == nc.ERR_MALLOC
         finally:
             nc.lib().numc_cuda_debug_fail_malloc(0)
+
+
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("shape", [(640, 640, 640), (1, 9001, 1), (64, 5000, 64)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_gemm_reports_abandoned_waits(dt, shape):
+    """numc_cuda_gemm with a workspace: one K split and several (which add into a
+    cleared output)."""
+    M, K, N = shape
+    a, b = _rand(dt, (M, K), 7), _rand(dt, (K, N), 8)
+    ta, tb = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    need = nc.workspace_size(dt, nc.ALGO_DEFAULT, -1, M, K, N)
+    if not need:
+        pytest.skip("the CUDA cores take this problem")
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    out = torch.zeros((M, N), dtype=ta.dtype, device="cuda")
+    with starved_waits():
+        nc.gemm(ta, tb, out, workspace=ws)
+        _internal(nc.check_status)
+    nc.check_status()
+    nc.gemm(ta, tb, out, workspace=ws)
+    nc.check_status()
+    np.testing.assert_array_equal(out.cpu().numpy(), oracle.matmul(a, b))
+
+
+def test_captured_call_takes_the_cuda_cores():
+    """A graph outlives the scratch of the calls captured in it: no digits there."""
+    n = 1024
+    a, b = _rand("int32", (n, n), 9), _rand("int32", (n, n), 10)
+    with nc.Ctx() as ctx:
+        A, B, Z = ctx.from_numpy(a), ctx.from_numpy(b), ctx.zeros((n, n), "int32")
+        C = ctx.zeros((n, n), "int32")
+        for t in (A, B, Z, C):
+            t.to_device()
+        nc.matmul(A, B, C)
+        ctx.synchronize()
+        g = torch.cuda.CUDAGraph()
+        k = nc.launch_count()
+        with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(ctx.stream())):
+            nc.matmul(A, B, C)
+        assert nc.launch_count() - k == 1
+        nc.matmul(Z, B, C)              # zeros in the output
+        ctx.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        C.to_host()
+        np.testing.assert_array_equal(C.numpy(), oracle.matmul(a, b))
