@@ -126,7 +126,7 @@ __device__ __forceinline__ void load8(const T *row, int64_t rs_k, int64_t k0, in
 // chunks), a block 64 rows x 32 k.  Contiguous rows are read as whole 128- or
 // 256-byte lines, row-contiguous operands (B, read as B^T) as 8-element
 // segments that fill sectors; per digit a warp writes two runs of 256 bytes.
-// Blocks past both operands' clear C for a K-split GEMM that adds into it.
+// Every block clears its share of C for a K-split GEMM that adds into it.
 template <typename T, int S>
 __global__ void __launch_bounds__(256)
 int_digits(DigitOperand a, DigitOperand b, int64_t K, int64_t Ks, unsigned kgroups,

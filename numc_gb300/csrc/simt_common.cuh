@@ -497,12 +497,13 @@ __host__ __device__ inline int64_t float_edge_groups(int64_t M, int64_t N, int i
 // FMA chain from zero, the block sums added in K order (numc's remainder
 // tiles).  Lanes past the last column return.
 // One numc K block of an output as an FMA chain from zero, k = pc .. pe-1
-// in order.  The operands are fetched U steps ahead into registers so the
-// chain waits for memory once per U steps, not once per step (32 for the
-// few-output, latency-bound fix-up: 232 registers a thread).
-template <typename T, int U>
+// in order.  The operands are fetched 32 steps ahead into registers so the
+// chain waits for memory once per 32 steps, not once per step (for the
+// few-output, latency-bound fix-up; 232 registers a thread).
+template <typename T>
 __device__ __forceinline__ T chain_block(const T *A, int64_t csa, const T *B, int64_t rsb,
                                          int64_t pc, int64_t pe) {
+  constexpr int U = 32;
   T t = T(0);
 #pragma unroll 1
   for (int64_t k0 = pc; k0 < pe; k0 += U) {
@@ -557,7 +558,7 @@ constexpr int kEdgeLanes = 8;
 // accumulation with the blocks computed in parallel.  Every lane of the
 // warp calls this with the same K (the fold shuffles across the warp);
 // `valid` is false for lanes past the last output.
-template <typename T, int U = 32>
+template <typename T>
 __device__ __forceinline__ void float_edge_output_lanes(const Gemm &g, int64_t e, bool valid, int64_t r0,
                                                   int64_t c0) {
   const int lane = threadIdx.x & 31, sub = lane & (kEdgeLanes - 1), base = lane & ~(kEdgeLanes - 1);
@@ -581,7 +582,7 @@ __device__ __forceinline__ void float_edge_output_lanes(const Gemm &g, int64_t e
     T t = T(0);
     if (valid && kb < nkb) {
       const int64_t pc = kb * kNumcKC, pe = min(pc + (int64_t)kNumcKC, g.K);
-      t = chain_block<T, U>(A, g.csa, B, g.rsb, pc, pe);
+      t = chain_block<T>(A, g.csa, B, g.rsb, pc, pe);
     }
 #pragma unroll
     for (int q = 0; q < kEdgeLanes; q++) {

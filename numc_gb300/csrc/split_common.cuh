@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "kernels.h"
 #include "status.h"
 #include "tc_common.cuh"
 
@@ -481,7 +482,7 @@ __host__ __device__ inline int staged_rows(int K) {
 // device under four blocks an SM (512^3 with 16 rows 13.5 us, with 8 13.1).
 inline int staged_rows_for(int K, int64_t total) {
   int rows = staged_rows(K);
-  while (rows > 8 && total / rows < 608) rows /= 2;
+  while (rows > 8 && total / rows < 4 * sm_count()) rows /= 2;
   return rows;
 }
 constexpr int kStagedFloats = 32 * 258 + 4;
