@@ -311,7 +311,8 @@ __device__ __forceinline__ void simt_tile(const Gemm &g, int rule8, int64_t m0, 
       int c = b_nfast ? e % BN : e / BK;
       int kk = b_nfast ? e / BN : e % BK;
       int64_t gj = n0 + c, gk = k0 + kk;
-      rb[q] = (gj < g.N && gk < g.K) ? widen<T, Acc>(B[gk * g.rsb + gj * g.csb]) : Acc(0);
+      // past K -0 (floats): A's 0 times it leaves any sum, -0 included, as it is
+      rb[q] = (gj < g.N && gk < g.K) ? widen<T, Acc>(B[gk * g.rsb + gj * g.csb]) : Acc(-0.0);
     }
   };
   auto store_tiles = [&](int buf) {

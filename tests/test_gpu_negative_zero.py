@@ -53,3 +53,42 @@ def test_plan():
         want = oracle.matmul(a.contiguous().cpu().numpy(), b.contiguous().cpu().numpy())
         assert out.cpu().numpy().tobytes() == want.tobytes()
     plan.free()
+
+
+@pytest.mark.parametrize("profile", PROFILES, ids=["x86", "neon"])
+@pytest.mark.parametrize("shape", [(20, 3, 20), (47, 45, 50), (130, 33, 130), (300, 100, 300),
+                                   (257, 300, 515), (1000, 513, 1000), (2100, 259, 1900)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_float64(shape, profile):
+    M, K, N = shape
+    a, b = np.full((M, K), -1e-200), np.full((K, N), 1e-200)
+    out = torch.full((M, N), float("nan"), dtype=torch.float64, device="cuda")
+    nc.gemm(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), out, algo=nc.ALGO_SIMT,
+            param=profile)
+    want = oracle.matmul(a, b, profile)
+    assert np.signbit(want).any()
+    assert out.cpu().numpy().tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("dt,tiny", [("float32", 1e-30), ("float64", 1e-200)])
+def test_naive(dt, tiny):
+    """numc_matmul_naive: products rounded to -0 and added to +0."""
+    M, K, N = 70, 45, 90
+    a, b = np.full((M, K), -tiny, dt), np.full((K, N), tiny, dt)
+    with nc.Ctx() as ctx:
+        A, B, C = ctx.from_numpy(a), ctx.from_numpy(b), ctx.zeros((M, N), dt)
+        nc.matmul_naive(A, B, C)
+        assert C.numpy().tobytes() == oracle.matmul(a, b, oracle.PROFILE_WRAP).tobytes()
+
+
+@pytest.mark.parametrize("K", [37, 300])
+def test_strides_beyond_32_bits(K):
+    """Strides that the float32 tiles' offsets do not hold: the general kernel."""
+    M, N, wide = 3, 20000, 1 << 24
+    a = torch.full((M, wide), -1e-30, device="cuda")[:, :K]
+    b = torch.full((K, N), 1e-30, device="cuda")
+    out = torch.full((M, N), float("nan"), device="cuda")
+    nc.gemm(a, b, out, algo=nc.ALGO_SIMT, param=nc.INT8_X86_AVX2)
+    want = oracle.matmul(a.contiguous().cpu().numpy(), b.cpu().numpy())
+    assert np.signbit(want).any()
+    assert out.cpu().numpy().tobytes() == want.tobytes()
