@@ -191,7 +191,8 @@ NUMC_API int numc_cuda_gemm_host(NumcDType dtype, const void *a, const void *b,
                                  intptr_t rso);
 
 /* Waits for `stream` and reports any kernel that gave up on a bounded
- * wait (NUMC_ERR_INTERNAL); clears the flag. */
+ * wait (NUMC_ERR_INTERNAL); clears the flag, and those of contexts' integer
+ * products that no call of theirs has reported yet. */
 NUMC_API int numc_cuda_check_status(void *stream);
 
 /* Testing aids for the failure paths (no counterpart in numc).

@@ -513,9 +513,9 @@ grouped_f32_small(const Prob *__restrict__ probs, const Tile *__restrict__ tiles
 // steps below K are multiplied.  Measured, us with 128 x 128 tiles of scalar FMAs
 // and a pass for the remainders before, and with these tiles and the 16 x 16 and 32 x
 // 32 ones now: plans of the plain algorithm, 64 problems of 16 to 1024 399 / 93,
-// 500 of 16 to 256 171 / 139, 16 of 512 to 2048 1597 / 1169, one of 2000^3 671 /
+// 500 of 16 to 256 171 / 108, 16 of 512 to 2048 1597 / 1169, one of 2000^3 671 /
 // 424, 8 of 100 to 200 37 / 13.5; the 573 small problems of a mixed plan (most K
-// below 64: instructions of start and store weigh as much as the FMAs) 361 / 327.
+// below 64: instructions of start and store weigh as much as the FMAs) 361 / 310.
 using TileBig = f32::F32Cfg<16, 8, 8, 8>;
 constexpr int kBigCtas = 3, kBigRing = 8;
 
